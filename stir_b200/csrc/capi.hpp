@@ -17,6 +17,7 @@
 #include "../../include/stir_b200.h"
 #include "geometry.hpp"
 #include "internal.hpp"
+#include "zframe.hpp"
 
 namespace b200 {
 size_t projector_smem_bytes(const ProjParams& p);
@@ -138,6 +139,15 @@ struct b200rt_projector {
   DevBuf<PathCElem> path_cmaj;
   DevBuf<int> path_col_starts;
   PathParams pparams{};
+  // z-frame projection (zframe.cu), in place of the column-staged one where it applies: use_paths and use_z
+  bool use_z = false;
+  DevBuf<ZRec> z_recs;
+  DevBuf<ZItemDev> z_items;
+  ZParams zparams{};
+  cudaMemPool_t z_pool = nullptr;  // padded images of calls in flight
+  std::vector<char> h_item_lead;   // the first of a path item's parts (groups of chains, further lines)
+  DevBuf<int> z_work;              // the allocation-free log-likelihood's work list and partial sums
+  DevBuf<double> z_partials;
   std::vector<int> h_item_view;  // basic view of each path item
   std::vector<PathItemDev> h_path_items;
   std::map<std::pair<int, int>, std::unique_ptr<DevBuf<int>>> path_lists;
@@ -191,6 +201,18 @@ const int* path_list(b200rt_projector& h, int subset, int nsub, int& count);
 const int* tof_group_list(b200rt_projector& h, int subset, int nsub, int& count);
 void forward_subset(b200rt_projector& h, const float* image, float* out, int subset, int nsub, cudaStream_t st,
                     const FwdEpilogue* ep = nullptr);
+bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std::vector<LineDev>& lines, int nviews,
+                  int nsegs, int ntangs, const std::vector<int>& bviews);
+// path-item projections of a list of items for a batch of images (use_paths).  n_call: the items of the whole call where
+// the list is a part of it (-1: the list is)
+void forward_paths(b200rt_projector& h, const int* list, int n, const float* images, int64_t img_stride, float* out,
+                   int64_t out_stride, int batch, cudaStream_t st, const FwdEpilogue* ep, bool may_alloc = true, int n_call = -1);
+void back_paths(b200rt_projector& h, const int* list, int n, const float* pd, int64_t pd_stride, float* images,
+                int64_t img_stride, int batch, cudaStream_t st, int zero_ends);
+void add_back_paths(b200rt_projector& h, const int* list, int n, const float* pd, int64_t pd_stride, float* images,
+                    int64_t img_stride, int batch, cudaStream_t st, int zero_ends);
+void back_paths_fixed(b200rt_projector& h, const int* list, int n, const float* pd, unsigned long long* acc,
+                      const double* scale, cudaStream_t st, int zero_ends);
 const int* subset_views(b200rt_projector& h, int subset, int nsub, int& count);
 void prior_weights(const Geometry& g, int only_2D, float w[27]);
 void back_project_into(b200rt_projector& h, const float* pd, float* image, int subset, int nsub, int mode, int zero_ends,

@@ -26,6 +26,9 @@ struct b200rt_batch {
     b200rt_prior prior{};
     float prior_w[27] = {0};
     float min_rel = 0.f, max_rel = 0.f;
+    // z-frame geometries: the estimate in padded columns, made before the forward projection, and the numerator (not of
+    // deterministic frames), copied to u after the back projection
+    DevBuf<float> xpad, upad;
     DevBuf<float> ratio, u, grad, small_value, partial_max, umax;
     DevBuf<unsigned int> cancelled;
     // B200RT_BACKPROJECT_DETERMINISTIC: fixed-point numerator, its scale (from the ratio's bound 1e4 and the
@@ -41,13 +44,21 @@ struct b200rt_batch {
   std::vector<b200rt_projector*> geoms;
   DevBuf<b200::ProjParams> d_geoms;
   DevBuf<b200::PathParams> d_pgeoms;
+  DevBuf<b200::ZParams> d_zgeoms;
+  // kernels of the path-item family: the column-staged one (z = -1) and the z-frame variants the geometries use, each
+  // with its shared memory and most persistent CTAs per SM (forward, back)
+  struct PathKernel {
+    int z;  // a geometry of the variant
+    int smem[2], max_ctas[2];
+  };
+  std::vector<PathKernel> path_kernels;
+  std::vector<int> geom_kernel;  // geometry -> entry of path_kernels
   // kernel families (index B200RT_BATCH_KERNELS_*) the frames allow, the one in use, and each one's most
   // persistent CTAs per SM (forward, back)
   bool avail[5] = {false, false, false, false, false};
   int family = B200RT_BATCH_KERNELS_PATHS;
   int max_f[5] = {0, 0, 0, 0, 0}, max_b[5] = {0, 0, 0, 0, 0};
   int num_tof = 1;
-  int smem_f = 0, smem_b = 0;
   DevBuf<b200::BatchFrameDev> d_frames;
   DevBuf<unsigned int> counters;  // work-queue heads of the forward and back launches
   bool ready = false;
@@ -58,6 +69,11 @@ struct b200rt_batch {
   // item lists by (order, subset of each frame or -1)
   std::map<std::vector<int>, std::unique_ptr<DevBuf<b200::BatchItem>>> items;
   std::map<std::vector<int>, int> item_counts;
+  // the path-item family's lists, kernel by kernel: (entry of path_kernels, first item, items)
+  struct Part {
+    int kernel, first, count;
+  };
+  std::map<std::vector<int>, std::vector<Part>> item_parts;
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
   // per batched sub-iteration: the update arguments of its frames (device table), their count, the most blocks
   std::map<int, std::unique_ptr<DevBuf<b200::BatchUpdateDev>>> updates;
@@ -129,16 +145,34 @@ void batch_finalize(b200rt_batch& b) {
   b.avail[B200RT_BATCH_KERNELS_BASIC_BINS] = !deterministic;
   if (paths) {
     std::vector<b200::PathParams> pg;
-    b.smem_f = b.smem_b = 0;
-    for (auto* h : b.geoms) {
+    std::vector<b200::ZParams> zg;
+    b.path_kernels.clear();
+    b.geom_kernel.clear();
+    for (size_t gi = 0; gi < b.geoms.size(); ++gi) {
+      const b200rt_projector* h = b.geoms[gi];
       const b200::PathParams& pp = h->pparams;
       pg.push_back(pp);
-      b.smem_f = std::max(b.smem_f, b200::path_smem_fwd(pp.K, h->params.nz, pp.zpad, pp.max_lines, pp.max_acc,
-                                                          pp.npa_max).total);
-      b.smem_b = std::max(b.smem_b, b200::path_smem_back(h->params.nz, pp.max_lines, pp.max_members, pp.nax_max,
-                                                          pp.npa_max).total);
+      zg.push_back(h->zparams);
+      int smem[2];
+      if (h->use_z) {
+        smem[0] = b200::z_batch_smem(h->zparams, true);
+        smem[1] = b200::z_batch_smem(h->zparams, false);
+      } else {
+        smem[0] = b200::path_smem_fwd(pp.K, h->params.nz, pp.zpad, pp.max_lines, pp.max_acc, pp.npa_max).total;
+        smem[1] = b200::path_smem_back(h->params.nz, pp.max_lines, pp.max_members, pp.nax_max, pp.npa_max).total;
+      }
+      size_t k = 0;
+      for (; k < b.path_kernels.size(); ++k) {
+        const int zi = b.path_kernels[k].z;
+        if (h->use_z ? zi >= 0 && b200::z_same_variant(b.geoms[zi]->zparams, h->zparams) : zi < 0) break;
+      }
+      if (k == b.path_kernels.size())
+        b.path_kernels.push_back({h->use_z ? static_cast<int>(gi) : -1, {0, 0}, {0, 0}});
+      for (int d = 0; d < 2; ++d) b.path_kernels[k].smem[d] = std::max(b.path_kernels[k].smem[d], smem[d]);
+      b.geom_kernel.push_back(static_cast<int>(k));
     }
     b.d_pgeoms.upload(pg, st);
+    b.d_zgeoms.upload(zg, st);
   }
   std::vector<BatchFrameDev> fd;
   for (auto& fp : b.frames) {
@@ -168,7 +202,16 @@ void batch_finalize(b200rt_batch& b) {
       ensure_colmax(*f.h, f.u.p, st);
       ck(launch_fixed_scale(f.bound.p, 1, f.h->colmax.p, f.det_partial.p, f.fixed_scale.p, st), "scale");
     }
+    const size_t padded = static_cast<size_t>(b200::z_stride(f.h->zparams)) * g.desc().ny * g.desc().nx;
+    f.xpad.release();
+    f.upad.release();
+    if (paths && f.h->use_z && f.h->zparams.planes > 1) {
+      f.xpad.alloc(padded);
+      if (f.mode != B200RT_BACKPROJECT_DETERMINISTIC) f.upad.alloc(padded);
+    }
     BatchFrameDev d{};
+    d.xpad = f.xpad.p;
+    d.upad = f.upad.p;
     d.geom = f.geom;
     d.x = f.x;
     d.ratio = f.ratio.p;
@@ -184,11 +227,20 @@ void batch_finalize(b200rt_batch& b) {
     fd.push_back(d);
   }
   b.d_frames.upload(fd, st);
-  b.counters.alloc(2);
+  b.counters.alloc(2 * std::max<size_t>(1, b.path_kernels.size()));  // per kernel and direction
   ck(cudaDeviceGetAttribute(&b.num_sms, cudaDevAttrMultiProcessorCount, b.device), "device attribute");
   if (b.avail[B200RT_BATCH_KERNELS_PATHS]) {
-    b.max_f[B200RT_BATCH_KERNELS_PATHS] = b200::batch_paths_max_ctas_per_sm(b.npa, b.smem_f, true);
-    b.max_b[B200RT_BATCH_KERNELS_PATHS] = b200::batch_paths_max_ctas_per_sm(b.npa, b.smem_b, false);
+    int most[2] = {0, 0};
+    bool fits = true;
+    for (auto& k : b.path_kernels)
+      for (int d = 0; d < 2; ++d) {
+        k.max_ctas[d] = k.z < 0 ? b200::batch_paths_max_ctas_per_sm(b.npa, k.smem[d], d == 0)
+                                : b200::z_batch_max_ctas_per_sm(b.geoms[k.z]->zparams, d == 0, k.smem[d]);
+        most[d] = std::max(most[d], k.max_ctas[d]);
+        fits = fits && k.max_ctas[d] > 0;
+      }
+    b.max_f[B200RT_BATCH_KERNELS_PATHS] = fits ? most[0] : 0;
+    b.max_b[B200RT_BATCH_KERNELS_PATHS] = fits ? most[1] : 0;
   }
   if (b.avail[B200RT_BATCH_KERNELS_TOF_GROUPED]) {
     b.max_f[B200RT_BATCH_KERNELS_TOF_GROUPED] = b200::batch_tof_max_ctas_per_sm(b.num_tof, true);
@@ -209,10 +261,15 @@ void batch_finalize(b200rt_batch& b) {
   b.ready = true;
 }
 
-// the (frame, basic bin) work of batched sub-iteration k, uploaded on first use
-const BatchItem* batch_items(b200rt_batch& b, int k, int order, int& count) {
+std::vector<int> item_key(const b200rt_batch& b, int k, int order) {
   std::vector<int> key{order, b.family};
   for (auto& f : b.frames) key.push_back(k <= f->num_subiters ? frame_subset(*f, k) : -1);
+  return key;
+}
+
+// the (frame, basic bin) work of batched sub-iteration k, uploaded on first use
+const BatchItem* batch_items(b200rt_batch& b, int k, int order, int& count) {
+  const std::vector<int> key = item_key(b, k, order);
   auto it = b.items.find(key);
   if (it != b.items.end()) {
     count = b.item_counts[key];
@@ -251,6 +308,22 @@ const BatchItem* batch_items(b200rt_batch& b, int k, int order, int& count) {
     }
     per_frame[fi] = std::move(bins);
   }
+  // the frame's entries of the list, in units of `unit` that stay together: z-frame kernels take kZWarps items a CTA, or
+  // one item kZWarps times where the frame's own call would share it between the warps (z_parts)
+  std::vector<std::vector<BatchItem>> entries(b.frames.size());
+  std::vector<size_t> unit(b.frames.size(), 1);
+  for (size_t fi = 0; fi < b.frames.size(); ++fi) {
+    const b200rt_projector& h = *b.frames[fi]->h;
+    const int frame = static_cast<int>(fi);
+    const bool zf = b.family == B200RT_BATCH_KERNELS_PATHS && h.use_z;
+    const int parts = zf ? b200::z_parts(h.zparams, static_cast<int>(per_frame[fi].size())) : 1;
+    for (int bin : per_frame[fi])
+      for (int q = 0; q < parts; ++q) entries[fi].push_back(BatchItem{frame | (parts > 1 ? b200::kZShared : 0), bin});
+    if (zf) {
+      unit[fi] = b200::kZWarps;
+      while (entries[fi].size() % b200::kZWarps) entries[fi].push_back(BatchItem{frame, -1});
+    }
+  }
   if (order == 2) {
     // item-major: frames of one geometry in the same subset take each work item in turn, so that its row is read
     // from HBM once for all of them
@@ -264,12 +337,24 @@ const BatchItem* batch_items(b200rt_batch& b, int k, int order, int& count) {
           group.push_back(fj);
           done[fj] = true;
         }
-      for (size_t i = 0; i < per_frame[fi].size(); ++i)
-        for (size_t fj : group) list.push_back(BatchItem{static_cast<int>(fj), per_frame[fj][i]});
+      for (size_t i = 0; i < entries[fi].size(); i += unit[fi])
+        for (size_t fj : group)
+          list.insert(list.end(), entries[fj].begin() + i, entries[fj].begin() + i + unit[fi]);
     }
   } else {
-    for (size_t fi = 0; fi < b.frames.size(); ++fi)
-      for (int bin : per_frame[fi]) list.push_back(BatchItem{static_cast<int>(fi), bin});
+    for (size_t fi = 0; fi < b.frames.size(); ++fi) list.insert(list.end(), entries[fi].begin(), entries[fi].end());
+  }
+  if (b.family == B200RT_BATCH_KERNELS_PATHS) {  // kernel by kernel, in the order above within each
+    std::vector<BatchItem> by;
+    std::vector<b200rt_batch::Part> parts;
+    for (size_t k = 0; k < b.path_kernels.size(); ++k) {
+      const int first = static_cast<int>(by.size());
+      for (const BatchItem& it : list)
+        if (b.geom_kernel[b.frames[it.frame & ~b200::kZShared]->geom] == static_cast<int>(k)) by.push_back(it);
+      parts.push_back({static_cast<int>(k), first, static_cast<int>(by.size()) - first});
+    }
+    list.swap(by);
+    b.item_parts[key] = std::move(parts);
   }
   auto buf = std::make_unique<DevBuf<BatchItem>>();
   buf->upload(list, b.capture_stream);
@@ -309,18 +394,48 @@ void batch_zero(b200rt_batch& b, int k, cudaStream_t st) {
     ck(cudaMemsetAsync(f.cancelled.p, 0, sizeof(unsigned int), st), "memset");
     if (f.mode == B200RT_BACKPROJECT_DETERMINISTIC)
       ck(cudaMemsetAsync(f.acc64.p, 0, sizeof(unsigned long long) * f.h->geo->image_size(), st), "memset");
+    else if (f.upad.p && b.family == B200RT_BATCH_KERNELS_PATHS)
+      ck(cudaMemsetAsync(f.upad.p, 0, sizeof(float) * f.upad.n, st), "memset");
     else
       ck(cudaMemsetAsync(f.u.p, 0, sizeof(float) * f.h->geo->image_size(), st), "memset");
   }
 }
 
+// the estimates of the frames taking part in sub-iteration k in padded columns
+void batch_pad(b200rt_batch& b, int k, cudaStream_t st) {
+  if (b.family != B200RT_BATCH_KERNELS_PATHS) return;
+  for (auto& fp : b.frames)
+    if (k <= fp->num_subiters && fp->xpad.p) {
+      const auto& d = fp->h->geo->desc();
+      ck(b200::launch_pad_image(fp->x, 0, fp->xpad.p, 0, static_cast<int64_t>(d.ny) * d.nx, d.nz,
+                                b200::z_stride(fp->h->zparams), 1, st),
+         "estimate");
+    }
+}
+
 // one batched launch of one direction (0 forward with the ratio epilogue, 1 back projection of the ratios)
-cudaError_t batch_launch(b200rt_batch& b, int dir, const BatchItem* items, int n, int grid, cudaStream_t st) {
-  if (b.family == B200RT_BATCH_KERNELS_PATHS)
-    return dir == 0 ? b200::launch_forward_batch_paths(b.d_geoms.p, b.d_pgeoms.p, b.npa, b.smem_f, b.d_frames.p, items,
-                                                       n, b.counters.p, grid, st)
-                    : b200::launch_back_batch_paths(b.d_geoms.p, b.d_pgeoms.p, b.smem_b, b.d_frames.p, items, n,
-                                                    b.counters.p + 1, grid, st);
+cudaError_t batch_launch(b200rt_batch& b, int dir, int k, int order, const BatchItem* items, int n, int grid,
+                         cudaStream_t st) {
+  if (b.family == B200RT_BATCH_KERNELS_PATHS) {
+    for (const auto& part : b.item_parts.at(item_key(b, k, order))) {
+      const auto& pk = b.path_kernels[part.kernel];
+      const int g = std::min(grid, pk.max_ctas[dir] * b.num_sms);
+      unsigned* counter = b.counters.p + 2 * part.kernel + dir;
+      const BatchItem* it = items + part.first;
+      cudaError_t e;
+      if (pk.z >= 0)
+        e = b200::launch_z_batch(b.geoms[pk.z]->zparams, dir == 0, b.d_geoms.p, b.d_zgeoms.p, b.d_frames.p, it,
+                                 part.count / b200::kZWarps, counter, pk.smem[dir], g, st);
+      else if (dir == 0)
+        e = b200::launch_forward_batch_paths(b.d_geoms.p, b.d_pgeoms.p, b.npa, pk.smem[0], b.d_frames.p, it, part.count,
+                                             counter, g, st);
+      else
+        e = b200::launch_back_batch_paths(b.d_geoms.p, b.d_pgeoms.p, pk.smem[1], b.d_frames.p, it, part.count, counter, g,
+                                          st);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  }
   if (b.family == B200RT_BATCH_KERNELS_TOF_GROUPED)
     return dir == 0 ? b200::launch_forward_batch_tof(b.d_geoms.p, b.num_tof, b.d_frames.p, items, n, b.counters.p, grid,
                                                      st)
@@ -337,9 +452,10 @@ cudaError_t batch_launch(b200rt_batch& b, int dir, const BatchItem* items, int n
 void batch_projections(b200rt_batch& b, int k, cudaStream_t st) {
   int n = 0;
   const BatchItem* items = batch_items(b, k, b.cfg.order, n);
-  ck(cudaMemsetAsync(b.counters.p, 0, 2 * sizeof(unsigned int), st), "memset");
-  ck(batch_launch(b, 0, items, n, grid_of(b, b.cfg.ctas_per_sm_forward, b.max_fwd), st), "batched forward projection");
-  ck(batch_launch(b, 1, items, n, grid_of(b, b.cfg.ctas_per_sm_back, b.max_back), st), "batched back projection");
+  ck(cudaMemsetAsync(b.counters.p, 0, b.counters.n * sizeof(unsigned int), st), "memset");
+  batch_pad(b, k, st);
+  ck(batch_launch(b, 0, k, b.cfg.order, items, n, grid_of(b, b.cfg.ctas_per_sm_forward, b.max_fwd), st), "batched forward projection");
+  ck(batch_launch(b, 1, k, b.cfg.order, items, n, grid_of(b, b.cfg.ctas_per_sm_back, b.max_back), st), "batched back projection");
 }
 
 // the update arguments of the frames taking part in sub-iteration k, uploaded on first use
@@ -379,6 +495,14 @@ void batch_subiteration(b200rt_batch& b, int k, cudaStream_t st) {
   for (auto& fp : b.frames)  // deterministic frames: their fixed-point numerators to float
     if (k <= fp->num_subiters && fp->mode == B200RT_BACKPROJECT_DETERMINISTIC)
       ck(launch_fixed_to_float(fp->acc64.p, fp->fixed_scale.p, fp->u.p, fp->h->geo->image_size(), st), "numerator");
+  if (b.family == B200RT_BATCH_KERNELS_PATHS)  // numerators in padded columns to the image's
+    for (auto& fp : b.frames)
+      if (k <= fp->num_subiters && fp->upad.p) {
+        const auto& d = fp->h->geo->desc();
+        ck(b200::launch_unpad_image(fp->upad.p, 0, fp->u.p, 0, static_cast<int64_t>(d.ny) * d.nx, d.nz,
+                                    b200::z_stride(fp->h->zparams), 1, st),
+           "numerator");
+      }
   // every frame's update (OSMAPOSLReconstruction.cxx:394-510) in three launches
   int n = 0, max_blocks = 1;
   const b200::BatchUpdateDev* upd = batch_updates(b, k, n, max_blocks);
@@ -421,6 +545,7 @@ void b200rt_batch_destroy(b200rt_batch* b) {
     b->frames.clear();
     b->d_geoms.release();
     b->d_pgeoms.release();
+    b->d_zgeoms.release();
     b->d_frames.release();
     b->counters.release();
     if (b->capture_stream) cudaStreamDestroy(b->capture_stream);
@@ -487,6 +612,7 @@ int b200rt_batch_add_frame(b200rt_batch* b, b200rt_projector* h, float* estimate
     b->updates.clear();
     b->update_counts.clear();
     b->item_counts.clear();
+    b->item_parts.clear();
     b->ready = false;
     b->frames.push_back(std::move(f));
     if (frame) *frame = static_cast<int>(b->frames.size()) - 1;
@@ -558,12 +684,12 @@ int b200rt_batch_autotune(b200rt_batch* b, int subiteration, b200rt_batch_config
     batch_thresholds(*b, subiteration, st);  // the forward epilogue reads them
     batch_zero(*b, subiteration, st);        // numerators are scratch
     // time one launch of one direction: the best of two after a warm-up
-    auto time_launch = [&](int dir, const BatchItem* items, int n, int grid) {
+    auto time_launch = [&](int dir, int order, const BatchItem* items, int n, int grid) {
       float t = 1e30f;
       for (int rep = 0; rep < 3; ++rep) {
-        ck(cudaMemsetAsync(b->counters.p, 0, 2 * sizeof(unsigned int), st), "memset");
+        ck(cudaMemsetAsync(b->counters.p, 0, b->counters.n * sizeof(unsigned int), st), "memset");
         ck(cudaEventRecord(e0, st), "cudaEventRecord");
-        ck(batch_launch(*b, dir, items, n, grid, st), dir == 0 ? "batched forward projection" : "batched back projection");
+        ck(batch_launch(*b, dir, subiteration, order, items, n, grid, st), dir == 0 ? "batched forward projection" : "batched back projection");
         ck(cudaEventRecord(e1, st), "cudaEventRecord");
         ck(cudaEventSynchronize(e1), "cudaEventSynchronize");
         float ms = 0.f;
@@ -577,6 +703,7 @@ int b200rt_batch_autotune(b200rt_batch* b, int subiteration, b200rt_batch_config
     for (int fam = B200RT_BATCH_KERNELS_PATHS; fam <= B200RT_BATCH_KERNELS_BASIC_BINS; ++fam) {
       if (!b->avail[fam]) continue;
       use_family(*b, fam);
+      batch_pad(*b, subiteration, st);
       for (int order = 0; order <= 2; ++order) {
         if (order == 1 && fam == B200RT_BATCH_KERNELS_TOF_GROUPED) continue;  // TOF-grouped items: no length sort
         int n = 0;
@@ -585,7 +712,7 @@ int b200rt_batch_autotune(b200rt_batch* b, int subiteration, b200rt_batch_config
         int cdir[2] = {1, 1};
         for (int dir = 0; dir < 2; ++dir)
           for (int c = 1; c <= (dir == 0 ? b->max_fwd : b->max_back); ++c) {
-            const float t = time_launch(dir, items, n, c * b->num_sms);
+            const float t = time_launch(dir, order, items, n, c * b->num_sms);
             if (t < tdir[dir]) {
               tdir[dir] = t;
               cdir[dir] = c;

@@ -47,9 +47,7 @@ int b200rt_forward_project_batch_dev(b200rt_projector* h, const float* images_de
     if (h->use_paths) {
       int n = 0;
       const int* list = path_list(*h, subset_num, num_subsets, n);
-      ck(launch_forward_paths_batch(h->params, h->pparams, list, n, images_dev, image_stride, projdata_dev,
-                                    projdata_stride, batch, st, nullptr),
-         "forward projection");
+      forward_paths(*h, list, n, images_dev, image_stride, projdata_dev, projdata_stride, batch, st, nullptr);
     } else {
       for (int b = 0; b < batch; ++b)
         forward_subset(*h, images_dev + b * image_stride, projdata_dev + b * projdata_stride, subset_num, num_subsets, st);
@@ -71,14 +69,10 @@ int b200rt_back_project_batch_dev(b200rt_projector* h, const float* projdata_dev
   try {
     DeviceGuard dg(h->device);
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int64_t ni = h->geo->image_size();
     if (h->use_paths && back_projection_mode == B200RT_BACKPROJECT_ATOMIC) {
       int n = 0;
       const int* list = path_list(*h, subset_num, num_subsets, n);
-      for (int b = 0; b < batch; ++b) ck(cudaMemsetAsync(images_dev + b * image_stride, 0, sizeof(float) * ni, st), "memset");
-      ck(launch_back_paths_atomic_batch(h->params, h->pparams, list, n, projdata_dev, projdata_stride, images_dev,
-                                        image_stride, batch, st, 0),
-         "back projection");
+      back_paths(*h, list, n, projdata_dev, projdata_stride, images_dev, image_stride, batch, st, 0);
     } else {
       for (int b = 0; b < batch; ++b)
         back_project_into(*h, projdata_dev + b * projdata_stride, images_dev + b * image_stride, subset_num, num_subsets,
@@ -127,8 +121,7 @@ int b200rt_log_likelihood_batch_dev(b200rt_projector* h, const float* images_dev
     if (h->ll_partials.n < np) h->ll_partials.alloc(np);
     if (h->ll_sum.n < static_cast<size_t>(batch)) h->ll_sum.alloc(batch);
     ep.partials = h->ll_partials.p;
-    ck(launch_forward_paths_batch(h->params, h->pparams, list, n, images_dev, image_stride, nullptr, 0, batch, st, &ep),
-       "log-likelihood");
+    forward_paths(*h, list, n, images_dev, image_stride, nullptr, 0, batch, st, &ep);
     for (int b = 0; b < batch; ++b)
       ck(launch_reduce_sum(h->ll_partials.p + static_cast<int64_t>(b) * n, n, h->ll_sum.p + b, st), "reduce");
     ck(cudaMemcpyAsync(values, h->ll_sum.p, sizeof(double) * batch, cudaMemcpyDeviceToHost, st), "D2H");
@@ -173,9 +166,7 @@ int b200rt_log_likelihood_and_ratio_batch_dev(b200rt_projector* h, const float* 
     if (h->ll_partials.n < np) h->ll_partials.alloc(np);
     if (h->ll_sum.n < static_cast<size_t>(batch)) h->ll_sum.alloc(batch);
     ep.partials = h->ll_partials.p;
-    ck(launch_forward_paths_batch(h->params, h->pparams, list, n, images_dev, image_stride, ratio_dev, ratio_stride,
-                                  batch, st, &ep),
-       "log-likelihood");
+    forward_paths(*h, list, n, images_dev, image_stride, ratio_dev, ratio_stride, batch, st, &ep);
     for (int b = 0; b < batch; ++b)
       ck(launch_reduce_sum(h->ll_partials.p + static_cast<int64_t>(b) * n, n, h->ll_sum.p + b, st), "reduce");
     ck(cudaMemcpyAsync(values, h->ll_sum.p, sizeof(double) * batch, cudaMemcpyDeviceToHost, st), "D2H");
@@ -209,7 +200,6 @@ int b200rt_log_likelihood_gradient_batch_dev(b200rt_projector* h, const float* i
   }
   try {
     DeviceGuard dg(h->device);
-    const Geometry& g = *h->geo;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     int n = 0;
     const int* list = path_list(*h, subset_num, num_subsets, n);
@@ -233,14 +223,8 @@ int b200rt_log_likelihood_gradient_batch_dev(b200rt_projector* h, const float* i
     ep.cancelled = h->cancelled.p;
     ep.small_value = batch_thresholds(*h, y_dev, y_stride, batch, subset_num, num_subsets, zero_seg0_end_planes, st,
                                       ep.sv_stride);
-    ck(launch_forward_paths_batch(h->params, h->pparams, list, n, images_dev, image_stride, h->ratio_batch.p,
-                                  pd_size(*h), batch, st, &ep),
-       "forward projection");
-    for (int b = 0; b < batch; ++b)
-      ck(cudaMemsetAsync(gradients_dev + b * gradient_stride, 0, sizeof(float) * g.image_size(), st), "memset");
-    ck(launch_back_paths_atomic_batch(h->params, h->pparams, list, n, h->ratio_batch.p, pd_size(*h),
-                                      gradients_dev, gradient_stride, batch, st, 0),
-       "back projection");
+    forward_paths(*h, list, n, images_dev, image_stride, h->ratio_batch.p, pd_size(*h), batch, st, &ep);
+    back_paths(*h, list, n, h->ratio_batch.p, pd_size(*h), gradients_dev, gradient_stride, batch, st, 0);
     return B200RT_OK;
   } catch (const std::exception& e) {
     return fail(h, status_of(e), e.what());

@@ -66,6 +66,13 @@ __global__ void __launch_bounds__(1024) select_subset_kernel(const int* __restri
   }
 }
 
+// the same over the entries with lead[i] set
+int count_leads(const std::vector<int>& basic_view, const std::vector<char>& lead, int subset, int nsub) {
+  int c = 0;
+  for (size_t i = 0; i < basic_view.size(); ++i) c += lead[i] && basic_view[i] % nsub == subset;
+  return c;
+}
+
 int count_in_subset(const std::vector<int>& basic_view, int subset, int nsub) {
   int c = 0;
   for (int v : basic_view) c += v >= 0 && v % nsub == subset;
@@ -92,11 +99,14 @@ extern "C" int b200rt_log_likelihood_dev_noalloc(b200rt_projector* h, const floa
     const std::vector<int>& keys_h = h->use_paths ? h->h_item_view : grouped ? h->h_tof_basic_view : h->h_bin_view;
     const int* keys_d = h->use_paths ? h->item_view_dev.p : grouped ? h->tof_basic_view_dev.p : h->bin_view_dev.p;
     const int n = count_in_subset(keys_h, subset_num, num_subsets);
+    // z-frame items are parts of a path item: their lists and partial sums are the projector's own, made at set-up for
+    // all of them, and the limit counts path items
+    const int work = h->use_z ? count_leads(keys_h, h->h_item_lead, subset_num, num_subsets) : n;
     const int nv = count_in_subset(h->h_view_basic, subset_num, num_subsets);
     const int64_t nvg = static_cast<int64_t>(g.num_tof()) * (2 * g.S() + 1) * g.num_views();
-    if (n > kNoAllocMaxItems || nv > kNoAllocMaxViews || nvg > kNoAllocMaxViewgrams)
+    if (work > kNoAllocMaxItems || nv > kNoAllocMaxViews || nvg > kNoAllocMaxViewgrams)
       return fail(h, B200RT_ERR_TOO_LARGE,
-                  "b200rt_log_likelihood_dev_noalloc: the subset has " + std::to_string(n) + " work items (at most " +
+                  "b200rt_log_likelihood_dev_noalloc: the subset has " + std::to_string(work) + " work items (at most " +
                       std::to_string(kNoAllocMaxItems) + "), " + std::to_string(nv) + " views (at most " +
                       std::to_string(kNoAllocMaxViews) + "), and the data " + std::to_string(nvg) +
                       " viewgrams = " + std::to_string(g.num_tof()) + " timing bins x " +
@@ -107,10 +117,10 @@ extern "C" int b200rt_log_likelihood_dev_noalloc(b200rt_projector* h, const floa
       return B200RT_OK;
     }
     unsigned char* base = noalloc_scratch(h->device);
-    int* d_items = reinterpret_cast<int*>(base + kNoAllocItemsOff);
+    int* d_items = h->use_z ? h->z_work.p : reinterpret_cast<int*>(base + kNoAllocItemsOff);
     int* d_views = reinterpret_cast<int*>(base + kNoAllocViewsOff);
     float* d_small = reinterpret_cast<float*>(base + kNoAllocSmallOff);
-    double* d_partials = reinterpret_cast<double*>(base + kNoAllocPartialsOff);
+    double* d_partials = h->use_z ? h->z_partials.p : reinterpret_cast<double*>(base + kNoAllocPartialsOff);
     // every list entry, threshold and partial the kernels read is written by this call first
     select_subset_kernel<<<1, 1024, 0, st>>>(keys_d, static_cast<int>(keys_h.size()), subset_num, num_subsets,
                                              d_items);
@@ -129,7 +139,7 @@ extern "C" int b200rt_log_likelihood_dev_noalloc(b200rt_projector* h, const floa
     ep.small_value = d_small;
     ep.partials = d_partials;
     if (h->use_paths)
-      ck(launch_forward_paths(h->params, h->pparams, d_items, n, image_dev, nullptr, st, &ep), "log-likelihood");
+      forward_paths(*h, d_items, n, image_dev, 0, nullptr, 0, 1, st, &ep, false);
     else if (grouped)
       ck(launch_forward_tof_grouped(h->params, d_items, n, image_dev, nullptr, st, &ep), "log-likelihood");
     else

@@ -175,7 +175,7 @@ int b200rt_log_likelihood_dev(b200rt_projector* h, const float* image_dev, const
     ep.small_value = h->small_value.p;
     ep.partials = h->ll_partials.p;
     if (h->use_paths)
-      ck(launch_forward_paths(h->params, h->pparams, list, n, image_dev, nullptr, st, &ep), "log-likelihood");
+      forward_paths(*h, list, n, image_dev, 0, nullptr, 0, 1, st, &ep);
     else if (grouped)
       ck(launch_forward_tof_grouped(h->params, list, n, image_dev, nullptr, st, &ep), "log-likelihood");
     else

@@ -146,9 +146,8 @@ int b200rt_forward_project(b200rt_projector* h, const float* image_host, float* 
       for (size_t gi = 0; gi + 1 < vg.v0.size(); ++gi) {
         const int n = vg.off[gi + 1] - vg.off[gi];
         if (n > 0)
-          ck(launch_forward_paths(h->params, h->pparams, vg.list->p + vg.off[gi], n, h->st_img_b.p, h->st_pd_b.p, st,
-                                  nullptr),
-             "forward projection");
+          forward_paths(*h, vg.list->p + vg.off[gi], n, h->st_img_b.p, 0, h->st_pd_b.p, 0, 1, st, nullptr, true,
+                        vg.off.back());
         ck(projdata_layout_views(*h, h->st_pd_b.p, h->st_pd_a.p, false, vg.v0[gi], vg.v0[gi + 1], st), "layout");
         ck(cudaEventRecord(h->copy_events[gi], st), "cudaEventRecord");
         ck(cudaStreamWaitEvent(h->copy_stream, h->copy_events[gi], 0), "cudaStreamWaitEvent");
@@ -203,9 +202,7 @@ int b200rt_back_project(b200rt_projector* h, const float* projdata_host, float* 
         ck(projdata_layout_views(*h, h->st_pd_a.p, h->st_pd_b.p, true, vg.v0[gi], vg.v0[gi + 1], st), "layout");
         const int n = vg.off[gi + 1] - vg.off[gi];
         if (n > 0)
-          ck(launch_back_paths_atomic(h->params, h->pparams, vg.list->p + vg.off[gi], n, h->st_pd_b.p, h->st_img_b.p,
-                                      st, 0),
-             "back projection");
+          add_back_paths(*h, vg.list->p + vg.off[gi], n, h->st_pd_b.p, 0, h->st_img_b.p, 0, 1, st, 0);
       }
     } else {
       ck(cudaMemcpyAsync(h->st_pd_a.p, projdata_host, sizeof(float) * g.projdata_size(), cudaMemcpyHostToDevice, st),

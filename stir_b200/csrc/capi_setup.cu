@@ -626,8 +626,10 @@ void setup_projector(b200rt_projector& h) {
     }
     h.total_nnz = t;
     if (g.num_tof() == 1)
-      build_paths(h, hr, lines, static_cast<int>(bviews.size()), static_cast<int>(bsegs.size()),
-                  static_cast<int>(btangs.size()), bviews);
+      if (!build_zframe(h, hr, lines, static_cast<int>(bviews.size()), static_cast<int>(bsegs.size()),
+                        static_cast<int>(btangs.size()), bviews))
+        build_paths(h, hr, lines, static_cast<int>(bviews.size()), static_cast<int>(bsegs.size()),
+                    static_cast<int>(btangs.size()), bviews);
   }
   // the basic view of every entry of each work list (bins, TOF basic bins, path items) and of every view (-1: a
   // view no basic view reaches), on the device: the allocation-free entry point selects a subset's work and views
@@ -722,7 +724,7 @@ void forward_subset(b200rt_projector& h, const float* image, float* out, int sub
   int n = 0;
   if (h.use_paths && (!ep || ep->mode != kEpiLoglik)) {
     const int* list = path_list(h, subset, nsub, n);
-    ck(launch_forward_paths(h.params, h.pparams, list, n, image, out, st, ep), "forward projection");
+    forward_paths(h, list, n, image, 0, out, 0, 1, st, ep);
   } else if (h.params.tof_w && (!ep || ep->mode != kEpiLoglik)) {  // log-likelihood partials: see its entry point
     const int* list = tof_group_list(h, subset, nsub, n);
     ck(launch_forward_tof_grouped(h.params, list, n, image, out, st, ep), "forward projection");
@@ -794,9 +796,9 @@ void ensure_colmax(b200rt_projector& h, float* scratch, cudaStream_t st) {
   const int* all = h.use_paths ? path_list(h, 0, 1, nall)
                    : grouped   ? tof_group_list(h, 0, 1, nall)
                                : subset_list(h, 0, 1, nall);
-  ck(cudaMemsetAsync(scratch, 0, sizeof(float) * ni, st), "memset");
+  if (!h.use_paths) ck(cudaMemsetAsync(scratch, 0, sizeof(float) * ni, st), "memset");
   if (h.use_paths)
-    ck(launch_back_paths_atomic(h.params, h.pparams, all, nall, nullptr, scratch, st, 0), "column sums");
+    back_paths(h, all, nall, nullptr, 0, scratch, 0, 1, st, 0);
   else if (grouped)
     ck(launch_back_tof_grouped(h.params, all, nall, nullptr, scratch, nullptr, nullptr, st, 0), "column sums");
   else
@@ -815,9 +817,9 @@ void back_project_into(b200rt_projector& h, const float* pd, float* image, int s
                     : grouped   ? tof_group_list(h, subset, nsub, n)
                                 : subset_list(h, subset, nsub, n);
   if (mode == B200RT_BACKPROJECT_ATOMIC) {
-    ck(cudaMemsetAsync(image, 0, sizeof(float) * ni, st), "memset");
+    if (!h.use_paths) ck(cudaMemsetAsync(image, 0, sizeof(float) * ni, st), "memset");
     if (h.use_paths)
-      ck(launch_back_paths_atomic(h.params, h.pparams, list, n, pd, image, st, zero_ends), "back projection");
+      back_paths(h, list, n, pd, 0, image, 0, 1, st, zero_ends);
     else if (grouped)
       ck(launch_back_tof_grouped(h.params, list, n, pd, image, nullptr, nullptr, st, zero_ends), "back projection");
     else
@@ -839,8 +841,7 @@ void back_project_into(b200rt_projector& h, const float* pd, float* image, int s
   }
   ck(cudaMemsetAsync(h.acc64.p, 0, sizeof(unsigned long long) * ni, st), "memset");
   if (h.use_paths)
-    ck(launch_back_paths_fixed(h.params, h.pparams, list, n, pd, h.acc64.p, h.fixed_scale.p, st, zero_ends),
-       "back projection");
+    back_paths_fixed(h, list, n, pd, h.acc64.p, h.fixed_scale.p, st, zero_ends);
   else if (grouped)
     ck(launch_back_tof_grouped(h.params, list, n, pd, nullptr, h.acc64.p, h.fixed_scale.p, st, zero_ends),
        "back projection");
@@ -986,6 +987,10 @@ void b200rt_destroy(b200rt_projector* h) {
     h->ones.release();
     h->ossps_partial.release();
     h->ossps_minpos.release();
+    h->z_recs.release();
+    h->z_items.release();
+    h->z_work.release();
+    h->z_partials.release();
     h->path_elems.release();
     h->path_cols.release();
     h->path_lines.release();
@@ -1039,6 +1044,7 @@ void b200rt_destroy(b200rt_projector* h) {
       cudaStreamDestroy(h->copy_stream);
     }
     for (cudaEvent_t e : h->copy_events) cudaEventDestroy(e);
+    if (h->z_pool) cudaMemPoolDestroy(h->z_pool);  // after the frees in flight
     if (h->stream) cudaStreamDestroy(h->stream);
   }
   delete h;

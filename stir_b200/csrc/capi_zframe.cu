@@ -1,0 +1,540 @@
+// Set-up of the z-frame tables and the dispatch between the two path-item projections (z-frame, column-staged).
+#include "capi.hpp"
+
+using namespace b200;
+
+namespace {
+
+// a chain of one member: per column its element before the event (w1), whether it moves up there, and the element after
+struct Chain {
+  int member;
+  int cur, z0;  // stored plane (z + 512) now and at the first column
+};
+
+struct Group {
+  std::vector<std::vector<ZRec>> recs;               // per chain group
+  std::vector<std::vector<int>> chain_member;        // per chain group: the member of every chain
+  std::vector<std::vector<int>> chain_z0, chain_z1;  // planes (z + 512) at the first column and at the end
+  bool ok = true;
+};
+
+// An event from stored plane zr to zr + 1 of a line (zt: plane of axial position 0 before it; dz: its move, 1 or -1):
+// the axial position that leaves the planes [0, planes), or -1, and whether one enters
+void edge_event(int zt, int dz, int nax, int npa, int planes, int& leave, bool& enters) {
+  auto at = [&](int d) { return d >= 0 && d % npa == 0 && d / npa < nax ? d / npa : -1; };
+  leave = dz > 0 ? at(planes - 1 - zt) : at(-zt);
+  enters = (dz > 0 ? at(-(zt + 1)) : at(planes - 1 - (zt - 1))) >= 0;
+}
+
+}  // namespace
+
+namespace capi {
+
+// The chains and records of every path (zframe.hpp).  Returns false, leaving no tables, where the z-frame kernels do not
+// apply: more than 128 planes, a column outside the image, or a basic bin with more chains than a warp takes.
+bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std::vector<LineDev>& lines, int nviews,
+                  int nsegs, int ntangs, const std::vector<int>& bviews) {
+  const Geometry& g = *h.geo;
+  const ProjParams& p = h.params;
+  if (g.num_tof() != 1 || p.nz < 1) return false;
+  ZParams z{};
+  if (p.nz > 128) return false;  // more planes than a warp holds
+  z.planes = p.nz <= 32 ? 1 : p.nz <= 64 ? 2 : 4;
+  const int64_t padded = static_cast<int64_t>(z_stride(z)) * p.ny * p.nx;
+  if (padded >= (int64_t(1) << 31)) return false;
+  const int ngroups = nviews * ntangs;
+  const int planes = 32 * z.planes;
+
+  struct Elem {
+    int z;
+    float v;
+  };
+  // pass 0 counts the chains a path needs, pass 1 builds the records for groups of z.nm chains
+  std::vector<Group> groups(ngroups);
+  std::vector<int> chains_of(ngroups, 0), chains_max(ngroups, 0);
+  auto work = [&](int g0, int g1, int cap) {
+    std::vector<uint32_t> keys;
+    std::vector<int> order;
+    for (int gi = g0; gi < g1; ++gi) {
+      Group& G = groups[gi];
+      try {
+        const int vi = gi / ntangs, ti = gi % ntangs;
+        keys.clear();
+        for (int si = 0; si < nsegs; ++si) {
+          const ProjBinDev& pb = h.h_bins[(static_cast<size_t>(vi) * nsegs + si) * ntangs + ti];
+          for (int k = 0; k < pb.row_len; ++k) keys.push_back(hr[pb.row_offset + k].zyx & 0x3fffffu);  // x, y bits
+        }
+        std::sort(keys.begin(), keys.end());
+        keys.erase(std::unique(keys.begin(), keys.end()), keys.end());
+        const int ncols = static_cast<int>(keys.size());
+        // every member's elements by column, planes ascending within a column
+        std::vector<std::vector<std::vector<Elem>>> el(nsegs, std::vector<std::vector<Elem>>(ncols));
+        for (int si = 0; si < nsegs; ++si) {
+          const ProjBinDev& pb = h.h_bins[(static_cast<size_t>(vi) * nsegs + si) * ntangs + ti];
+          for (int k = 0; k < pb.row_len; ++k) {
+            const RowElem e = hr[pb.row_offset + k];
+            const size_t c = std::lower_bound(keys.begin(), keys.end(), e.zyx & 0x3fffffu) - keys.begin();
+            el[si][c].push_back(Elem{static_cast<int>(e.zyx >> 22), e.v});
+          }
+          for (auto& v : el[si])
+            std::stable_sort(v.begin(), v.end(), [](const Elem& a, const Elem& b) { return a.z < b.z; });
+        }
+        // the columns along the path: a ray steps in x or in y, so x + y (or x - y) orders them; away from the end where
+        // the steepest member's planes are higher
+        double mx = 0, my = 0, cov = 0;
+        for (uint32_t k : keys) mx += k & 2047u, my += k >> 11;
+        mx /= ncols, my /= ncols;
+        for (uint32_t k : keys) cov += ((k & 2047u) - mx) * ((k >> 11) - my);
+        const int sy = cov >= 0 ? 1 : -1;
+        auto along = [&](int c) { return static_cast<int>(keys[c] & 2047u) + sy * static_cast<int>(keys[c] >> 11); };
+        order.resize(ncols);
+        for (int c = 0; c < ncols; ++c) order[c] = c;
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return along(a) < along(b); });
+        {
+          double s0 = 0, s1 = 0, n0 = 0, n1 = 0;  // mean plane of the last member in the two halves
+          for (int i = 0; i < ncols; ++i)
+            for (const Elem& e : el[nsegs - 1][order[i]]) (i < ncols / 2 ? s0 : s1) += e.z, (i < ncols / 2 ? n0 : n1) += 1;
+          if (n0 > 0 && n1 > 0 && s0 / n0 > s1 / n1) std::reverse(order.begin(), order.end());
+        }
+        // chains: each element goes to the member's chain with the highest plane not above it (one element per plane)
+        struct Link {
+          int chain;
+          Elem e;
+        };
+        std::vector<std::vector<Chain>> chains(nsegs);
+        std::vector<std::vector<std::vector<Link>>> links(nsegs, std::vector<std::vector<Link>>(ncols));
+        int total = 0, most = 0;
+        for (int si = 0; si < nsegs; ++si) {
+          for (int i = 0; i < ncols; ++i)
+            for (const Elem& e : el[si][order[i]]) {
+              int best = -1;
+              for (int c = 0; c < static_cast<int>(chains[si].size()); ++c) {
+                const int cz = chains[si][c].cur;
+                // a chain that is at this plane already in this column has taken the element of a merged ray
+                if (cz <= e.z && (best < 0 || cz > chains[si][best].cur)) best = c;
+              }
+              if (best < 0) {
+                best = static_cast<int>(chains[si].size());
+                chains[si].push_back(Chain{si, e.z, e.z});
+              }
+              chains[si][best].cur = e.z;
+              links[si][i].push_back(Link{best, e});
+            }
+          // lines of an empty row are projected too (to 0): a chain without elements
+          if (chains[si].empty()) chains[si].push_back(Chain{si, 512, 512});
+          total += static_cast<int>(chains[si].size());
+          most = std::max(most, static_cast<int>(chains[si].size()));
+        }
+        chains_of[gi] = total;
+        chains_max[gi] = most;
+        if (cap == 0) continue;
+        // members into groups of at most cap chains, in order
+        std::vector<std::vector<int>> members;
+        int fill = cap + 1;
+        for (int si = 0; si < nsegs; ++si) {
+          const int n = static_cast<int>(chains[si].size());
+          if (fill + n > cap) {
+            members.emplace_back();
+            fill = 0;
+          }
+          members.back().push_back(si);
+          fill += n;
+        }
+        for (const auto& mem : members) {
+          std::vector<int> cm, cz0, first(nsegs, 0);
+          for (int si : mem) {
+            first[si] = static_cast<int>(cm.size());
+            for (const Chain& c : chains[si]) {
+              cm.push_back(si);
+              cz0.push_back(c.z0);
+            }
+          }
+          const int nc = static_cast<int>(cm.size());
+          std::vector<int> cur = cz0;
+          std::vector<ZRec> recs;
+          for (int i = 0; i < ncols; ++i) {
+            const size_t head = recs.size();
+            auto fresh = [&]() {
+              ZRec r{};
+              r.xy = keys[order[i]];
+              recs.push_back(r);
+            };
+            fresh();
+            for (int si : mem)
+              for (const Link& l : links[si][i]) {
+                const int m = first[si] + l.chain;
+                // up to the element's plane: one event a record, in further records of the column where one is not enough
+                size_t k = head;
+                while (cur[m] < l.e.z) {
+                  while (k < recs.size() && (recs[k].op & (1u << m))) ++k;
+                  if (k == recs.size()) fresh();
+                  recs[k].op |= 1u << m;
+                  // what leaves and enters: the same for every line of the member in one z orientation (checked)
+                  const ProjBinDev& pb = h.h_bins[(static_cast<size_t>(vi) * nsegs + si) * ntangs + ti];
+                  int leave[2] = {-2, -2};
+                  for (int q = 0; q < pb.num_lines; ++q) {
+                    const LineDev& L = lines[pb.first_line + q];
+                    const int d = (L.flags & 8) ? 1 : 0;
+                    const int zt = d ? L.q + 512 - p.min_z - cur[m] : cur[m] - 512 - p.min_z;
+                    int out = -1;
+                    bool in = false;
+                    edge_event(zt, d ? -1 : 1, g.nax(L.seg), g.npa(L.seg), planes, out, in);
+                    if (leave[d] != -2 && leave[d] != out) G.ok = false;
+                    leave[d] = out;
+                    if (out >= 0 || in) recs[k].op |= 1u << (6 + m);
+                  }
+                  recs[k].leave[m] = static_cast<int32_t>((static_cast<uint32_t>(std::max(leave[1], -1)) << 16) |
+                                                          (static_cast<uint32_t>(std::max(leave[0], -1)) & 0xffffu));
+                  ++cur[m];
+                }
+                // the element: before the column's events at the chain's first plane here, after the event otherwise
+                bool placed = false;
+                for (size_t q = recs.size(); q-- > head;)
+                  if (recs[q].op & (1u << m)) {
+                    recs[q].w2[m] += l.e.v;
+                    placed = true;
+                    break;
+                  }
+                if (!placed) recs[head].w1[2 * m] += l.e.v;
+              }
+          }
+          while (recs.size() % 4) {  // the kernels take four records at a time
+            ZRec r{};
+            r.xy = recs.back().xy;
+            recs.push_back(r);
+          }
+          for (ZRec& r : recs) {
+            for (int m = 0; m < nc; ++m) {
+              if (r.w1[2 * m] == 0.f) r.op |= kZGuard;
+              r.w1[2 * m + 1] = r.w1[2 * m];
+              if ((r.op >> m & 1u) && r.w2[m] == 0.f) r.op |= 1u << (6 + m);
+            }
+          }
+          G.recs.push_back(std::move(recs));
+          G.chain_member.push_back(std::move(cm));
+          G.chain_z0.push_back(std::move(cz0));
+          G.chain_z1.push_back(std::move(cur));
+        }
+      } catch (const std::exception&) {
+        G.ok = false;
+      }
+    }
+  };
+  const int nthreads = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
+  auto run = [&](int stride, int cap) {
+    std::vector<std::thread> pool;
+    for (int t = 0; t < nthreads; ++t)
+      pool.emplace_back([&, t] {
+        // interleaved: neighbouring paths cost about the same
+        for (int gi = t * stride; gi < ngroups; gi += nthreads * stride) work(gi, gi + 1, cap);
+      });
+    for (auto& th : pool) th.join();
+  };
+  // chains a warp takes (4 or 6), from a sample of the paths: as few groups of chains as possible, evenly filled
+  run(7, 0);
+  int total = 1, most = 1;
+  auto count = [&]() {
+    for (int gi = 0; gi < ngroups; ++gi) {
+      total = std::max(total, chains_of[gi]);
+      most = std::max(most, chains_max[gi]);
+    }
+  };
+  count();
+  if (most > kZChains) return false;
+  const int ng = (total + kZChains - 1) / kZChains;
+  z.nm = std::max((total + ng - 1) / ng, most) <= 4 ? 4 : kZChains;
+  run(1, z.nm);
+  count();
+  if (most > kZChains) return false;
+  if (most > z.nm) {  // a path outside the sample needs more
+    z.nm = kZChains;
+    for (Group& G : groups) G = Group{};
+    run(1, z.nm);
+  }
+  int64_t nrecs = 0;
+  for (int gi = 0; gi < ngroups; ++gi) {
+    if (!groups[gi].ok) return false;
+    for (const auto& r : groups[gi].recs) nrecs += static_cast<int64_t>(r.size());
+  }
+  if (nrecs >= (int64_t(1) << 31) - 64) return false;
+
+  std::vector<ZItemDev> items;
+  std::vector<int> item_view, item_out_view;
+  std::vector<char> item_lead;  // the first item of a (path, T)
+  std::vector<PathItemDev> path_items;
+  std::vector<char> led(static_cast<size_t>(ntangs));
+  std::vector<int> base(ngroups);
+  int64_t at = 0;
+  for (int gi = 0; gi < ngroups; ++gi) {
+    base[gi] = static_cast<int>(at);
+    for (const auto& r : groups[gi].recs) at += static_cast<int64_t>(r.size());
+  }
+  // items by (block of kZWarps tangential positions, view, T, chain group): the warps of a CTA take neighbouring paths,
+  // whose columns overlap in L1, the CTAs that run together share their paths' records, and the longest paths (through
+  // the middle of the field of view) come first
+  for (int t0 = 0; t0 < ntangs; t0 += kZWarps)
+    for (int vi = 0; vi < nviews; ++vi)
+      for (int T = 0; T < 8; ++T) {
+        const int t1 = std::min(t0 + kZWarps, ntangs);
+        std::fill(led.begin(), led.end(), 0);
+        size_t most_groups = 0;
+        for (int ti = t0; ti < t1; ++ti) most_groups = std::max(most_groups, groups[vi * ntangs + ti].recs.size());
+        for (size_t gr = 0; gr < most_groups; ++gr)
+          for (int ti = t0; ti < t1; ++ti) {
+            const Group& G = groups[vi * ntangs + ti];
+            if (gr >= G.recs.size()) continue;
+            int rec0 = base[vi * ntangs + ti];
+            for (size_t k = 0; k < gr; ++k) rec0 += static_cast<int>(G.recs[k].size());
+            const auto& cm = G.chain_member[gr];
+            // the k-th line of each orientation under T of every member
+            for (int k = 0;; ++k) {
+              ZItemDev it{};
+              it.rec0 = rec0;
+              it.nrec = static_cast<int>(G.recs[gr].size());
+              it.flags = T;
+              int out = 0, nl = 0, ov = -2;
+              for (int s = 0; s < 2 * kZChains; ++s) {
+                it.slot[s] = make_int2(-1, -1);
+                it.owner[s] = static_cast<int8_t>(s);
+              }
+              for (size_t m = 0; m < cm.size(); ++m) {
+                it.z0[m] = static_cast<int16_t>(G.chain_z0[gr][m]);
+                it.z1[m] = static_cast<int16_t>(G.chain_z1[gr][m]);
+                const int b = (vi * nsegs + cm[m]) * ntangs + ti;
+                const ProjBinDev& pb = h.h_bins[b];
+                int seen[2] = {0, 0};
+                for (int l = 0; l < pb.num_lines; ++l) {
+                  const LineDev& L = lines[pb.first_line + l];
+                  if ((L.flags & 7) != T) continue;
+                  const int d = (L.flags & 8) ? 1 : 0;
+                  if (seen[d]++ != k) continue;
+                  const int s = 2 * static_cast<int>(m) + d;
+                  it.slot[s] = make_int2(pb.first_line + l, b);
+                  bool own = true;
+                  for (size_t m2 = 0; m2 < m; ++m2)
+                    if (cm[m2] == cm[m]) {
+                      it.owner[s] = static_cast<int8_t>(2 * m2 + d);
+                      own = false;
+                      break;
+                    }
+                  if (own) {
+                    out += g.nax(L.seg);
+                    ++nl;
+                  }
+                  ov = ov == -2 ? L.view : ov == L.view ? ov : -1;
+                }
+              }
+              if (nl == 0) break;
+              for (int m = static_cast<int>(cm.size()); m < 8; ++m) it.z0[m] = it.z1[m] = 512;
+              // the back projection's buffer: every line's data with the zeros around them that its planes reach, the zeros
+              // between two lines shared; first the zeros of the slots without a line
+              const int nplanes = planes;
+              int bend = 0, bzeros = 0;
+              for (int s = 0; s < 2 * kZChains; ++s) {
+                if (it.slot[s].x >= 0) continue;
+                const size_t m = static_cast<size_t>(s / 2);
+                const int z0 = m < cm.size() ? G.chain_z0[gr][m] : 512, up = m < cm.size() ? G.chain_z1[gr][m] - z0 : 0;
+                // zt = z0 (slot 2 m) or -z0 at the first column (setup_slots), one up or down an event: read from `up`
+                // down to 0, or from 0 up
+                it.boff[s] = static_cast<int16_t>(s % 2 ? -z0 : z0 + up);
+                bzeros = std::max(bzeros, nplanes + up);
+              }
+              for (size_t m = 0; m < cm.size(); ++m)
+                for (int d = 0; d < 2; ++d) {
+                  const int s = 2 * static_cast<int>(m) + d;
+                  if (it.slot[s].x < 0 || it.owner[s] != s) continue;
+                  const LineDev& L = lines[it.slot[s].x];
+                  const int reach = (g.nax(L.seg) - 1) * g.npa(L.seg);
+                  int lo = 0, hi = 0;  // planes read below datum 0 and above the last one, by any chain of the line
+                  for (size_t m2 = m; m2 < cm.size(); ++m2) {
+                    if (cm[m2] != cm[m]) continue;
+                    for (int zr : {G.chain_z0[gr][m2], G.chain_z1[gr][m2]}) {
+                      const int zt = (L.flags & 8) ? L.q + 512 - p.min_z - zr : zr - 512 - p.min_z;
+                      lo = std::max(lo, zt);
+                      hi = std::max(hi, nplanes - 1 - zt - reach);
+                    }
+                  }
+                  const int at = bend + std::max(bzeros, lo);
+                  if (at + reach + hi > 30000) return false;
+                  it.boff[s] = static_cast<int16_t>(at);
+                  bend = at + reach + 1;
+                  bzeros = hi;
+                }
+              for (int s = 0; s < 2 * kZChains; ++s)
+                if (it.owner[s] != s) it.boff[s] = it.boff[static_cast<int>(it.owner[s])];
+              z.max_back = std::max(z.max_back, bend + bzeros);
+              z.max_out = std::max(z.max_out, out);
+              items.push_back(it);
+              item_view.push_back(bviews[vi]);
+              item_lead.push_back(!led[ti]);
+              led[ti] = 1;
+              item_out_view.push_back(ov);
+              PathItemDev pi{};
+              pi.ncols = it.nrec;
+              pi.num_lines = nl;
+              path_items.push_back(pi);
+            }
+            // every column inside the image under T
+            const int swap = T & 1, sx = (T & 2) ? -1 : 1, sy = (T & 4) ? -1 : 1;
+            for (const ZRec& r : G.recs[gr]) {
+              const int x = static_cast<int>(r.xy & 2047u) - 1024, y = static_cast<int>(r.xy >> 11) - 1024;
+              const int xi = (swap ? y : x) * sx - p.min_x, yi = (swap ? x : y) * sy - p.min_y;
+              if (xi < 0 || xi >= p.nx || yi < 0 || yi >= p.ny) return false;
+            }
+          }
+      }
+  if (items.empty()) return false;
+  if (kZWarps * (std::max(z.max_out, z.max_back) * 4 + 8192) > 200 * 1024) return false;
+
+  h.z_recs.alloc(static_cast<size_t>(nrecs) + 2 * kZBatch);  // batches are fetched whole
+  std::vector<ZRec> all(static_cast<size_t>(nrecs) + 2 * kZBatch);
+  for (int gi = 0; gi < ngroups; ++gi) {
+    size_t o = static_cast<size_t>(base[gi]);
+    for (auto& r : groups[gi].recs) {
+      std::copy(r.begin(), r.end(), all.begin() + o);
+      o += r.size();
+      std::vector<ZRec>().swap(r);
+    }
+  }
+  h.z_recs.upload(all, h.stream);
+  h.z_items.upload(items, h.stream);
+  h.dev_status.alloc(1);
+  ck(cudaMemsetAsync(h.dev_status.p, 0, sizeof(unsigned), h.stream), "memset");
+  ck(cudaStreamSynchronize(h.stream), "path tables");
+  int64_t ngrp = 0;
+  for (const Group& G : groups) ngrp += static_cast<int64_t>(G.recs.size());
+  z.mean_rec = static_cast<int>(nrecs / std::max<int64_t>(1, ngrp));
+  z.recs = h.z_recs.p;
+  z.items = h.z_items.p;
+  h.zparams = z;
+  h.z_work.alloc(items.size());
+  h.z_partials.alloc(items.size());
+  h.h_item_lead = std::move(item_lead);
+  h.h_item_view = std::move(item_view);
+  h.h_item_out_view = std::move(item_out_view);
+  h.h_path_items = std::move(path_items);
+  h.paths_view_split =
+      std::find(h.h_item_out_view.begin(), h.h_item_out_view.end(), -1) == h.h_item_out_view.end();
+  // padded images come from a pool of the handle's own, in stream order: calls on several streams or threads have their
+  // own, freed memory stays with the handle until it is destroyed
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = h.device;
+  ck(cudaMemPoolCreate(&h.z_pool, &props), "cudaMemPoolCreate");
+  uint64_t keep = UINT64_MAX;
+  ck(cudaMemPoolSetAttribute(h.z_pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
+  h.use_paths = h.use_z = true;
+  return true;
+}
+
+namespace {
+
+// device memory of one call, given back to the handle's pool in stream order
+struct PoolBuf {
+  float* p = nullptr;
+  cudaStream_t st;
+  PoolBuf(b200rt_projector& h, size_t n, cudaStream_t s) : st(s) {
+    if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), n * sizeof(float), h.z_pool, st) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;  // the kernels also take the plain image, more slowly
+    }
+  }
+  PoolBuf(const PoolBuf&) = delete;
+  ~PoolBuf() {
+    if (p) cudaFreeAsync(p, st);
+  }
+};
+
+constexpr size_t kPadLimit = size_t(1) << 28;  // floats of padded images at a time (1 GiB)
+
+}  // namespace
+
+void forward_paths(b200rt_projector& h, const int* list, int n, const float* images, int64_t img_stride, float* out,
+                   int64_t out_stride, int batch, cudaStream_t st, const FwdEpilogue* ep, bool may_alloc, int n_call) {
+  if (n <= 0 || batch <= 0) return;
+  if (!h.use_z) {
+    ck(launch_forward_paths_batch(h.params, h.pparams, list, n, images, img_stride, out, out_stride, batch, st, ep),
+       "forward projection");
+    return;
+  }
+  const ZParams& z = h.zparams;
+  const int parts = z_parts(z, n_call >= 0 ? n_call : n);
+  if (z.planes == 1 || !may_alloc) {
+    ck(launch_forward_z(h.params, z, list, n, parts, images, img_stride, 0, out, out_stride, batch, st, ep), "forward projection");
+    return;
+  }
+  const int64_t ncols = static_cast<int64_t>(h.params.ny) * h.params.nx, per = ncols * z_stride(z);
+  const int step = static_cast<int>(std::min<int64_t>(batch, std::max<int64_t>(1, static_cast<int64_t>(kPadLimit) / per)));
+  PoolBuf pad(h, static_cast<size_t>(per) * step, st);
+  for (int b = 0; b < batch; b += step) {
+    const int nb = std::min(step, batch - b);
+    FwdEpilogue e{};
+    if (ep) {
+      e = *ep;
+      e.y += b * e.y_stride;
+      if (e.add) e.add += b * e.add_stride;
+      if (e.mult) e.mult += b * e.mult_stride;
+      if (e.small_value) e.small_value += b * e.sv_stride;
+      if (e.partials) e.partials += static_cast<int64_t>(b) * n;
+    }
+    const float* x = images + b * img_stride;
+    float* o = out ? out + b * out_stride : nullptr;
+    if (pad.p) {
+      ck(launch_pad_image(x, img_stride, pad.p, per, ncols, h.params.nz, z_stride(z), nb, st), "image planes");
+      ck(launch_forward_z(h.params, z, list, n, parts, pad.p, per, 1, o, out_stride, nb, st, &e), "forward projection");
+    } else {
+      ck(launch_forward_z(h.params, z, list, n, parts, x, img_stride, 0, o, out_stride, nb, st, &e), "forward projection");
+    }
+  }
+}
+
+// image b (overwritten) = the back projection of the list's items from projection data b
+void back_paths(b200rt_projector& h, const int* list, int n, const float* pd, int64_t pd_stride, float* images,
+                int64_t img_stride, int batch, cudaStream_t st, int zero_ends) {
+  const int64_t ni = h.geo->image_size();
+  if (h.use_z && h.zparams.planes > 1 && n > 0) {
+    const ZParams& z = h.zparams;
+    const int parts = z_parts(z, n);
+    const int64_t ncols = static_cast<int64_t>(h.params.ny) * h.params.nx, per = ncols * z_stride(z);
+    const int step =
+        static_cast<int>(std::min<int64_t>(batch, std::max<int64_t>(1, static_cast<int64_t>(kPadLimit) / per)));
+    PoolBuf pad(h, static_cast<size_t>(per) * step, st);
+    if (pad.p) {
+      for (int b = 0; b < batch; b += step) {
+        const int nb = std::min(step, batch - b);
+        ck(cudaMemsetAsync(pad.p, 0, sizeof(float) * per * nb, st), "memset");
+        ck(launch_back_z(h.params, z, list, n, parts, pd ? pd + b * pd_stride : nullptr, pd_stride, pad.p, per, 1, nb, st,
+                         zero_ends),
+           "back projection");
+        ck(launch_unpad_image(pad.p, per, images + b * img_stride, img_stride, ncols, h.params.nz, z_stride(z), nb, st),
+           "image planes");
+      }
+      return;
+    }
+  }
+  for (int b = 0; b < batch; ++b) ck(cudaMemsetAsync(images + b * img_stride, 0, sizeof(float) * ni, st), "memset");
+  add_back_paths(h, list, n, pd, pd_stride, images, img_stride, batch, st, zero_ends);
+}
+
+// the same, added to the images
+void add_back_paths(b200rt_projector& h, const int* list, int n, const float* pd, int64_t pd_stride, float* images,
+                    int64_t img_stride, int batch, cudaStream_t st, int zero_ends) {
+  if (n <= 0) return;
+  if (h.use_z)
+    ck(launch_back_z(h.params, h.zparams, list, n, z_parts(h.zparams, n), pd, pd_stride, images, img_stride, 0, batch, st, zero_ends),
+       "back projection");
+  else
+    ck(launch_back_paths_atomic_batch(h.params, h.pparams, list, n, pd, pd_stride, images, img_stride, batch, st, zero_ends),
+       "back projection");
+}
+
+void back_paths_fixed(b200rt_projector& h, const int* list, int n, const float* pd, unsigned long long* acc,
+                      const double* scale, cudaStream_t st, int zero_ends) {
+  if (h.use_z)
+    ck(launch_back_z_fixed(h.params, h.zparams, list, n, z_parts(h.zparams, n), pd, acc, scale, st, zero_ends), "back projection");
+  else
+    ck(launch_back_paths_fixed(h.params, h.pparams, list, n, pd, acc, scale, st, zero_ends), "back projection");
+}
+
+}  // namespace capi

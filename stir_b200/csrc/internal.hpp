@@ -133,6 +133,9 @@ struct BatchFrameDev {
   // deterministic back projection of this frame: 64-bit fixed-point sums and their scale (null: float atomics)
   unsigned long long* acc64;
   const double* fixed_scale;
+  // z-frame geometries with several planes per lane: the estimate and the numerator in padded columns
+  const float* xpad;
+  float* upad;
 };
 struct BatchItem {
   int frame;

@@ -1,0 +1,91 @@
+// Tables and launchers of the z-frame projections (zframe.cu).
+//
+// A path item is a transaxial path (basic view, tangential position) under one transaxial symmetry operation, with the
+// lines of all its basic segments in both z orientations.  Its rows are cut into chains: along the path a chain has at
+// most one element per column and plane, and its plane never decreases, so that a register file which holds a line's
+// sums (or data) in image planes has to be moved by one plane only where the chain crosses one (an event).
+#pragma once
+
+#include "internal.hpp"
+
+namespace b200 {
+
+constexpr int kZChains = 6;      // chains of an item (one warp); more go to further items of the path
+constexpr int kZBatch = 8;       // records staged at a time
+constexpr int kZWarps = 4;       // items (warps) per CTA
+
+// One column of the path for every chain of the group: w1 before the column's events, w2 after them.
+struct __align__(16) ZRec {
+  float w1[2 * kZChains];  // each twice: the packed multiply-adds take pairs
+  float w2[kZChains];
+  int32_t leave[kZChains];  // forward: the axial positions of the up (low half) and down line whose sums leave the planes
+                            // at the event, -1: none
+  uint32_t xy;   // (x + 1024) | (y + 1024) << 11
+  uint32_t op;   // bits 0..5: chain m moves up one plane (its event); 6..11: that event needs the edge code (a position
+                 // leaves or enters the planes, or w2 is 0);
+                 // bit 12: some w1 is 0 (that product is left out: 0 x inf would make a NaN)
+  uint32_t pad[2];
+};
+static_assert(sizeof(ZRec) == 112, "a record is seven 16-byte pieces");
+constexpr uint32_t kZGuard = 1u << 12;
+
+// slot 2 m: the line of chain m whose planes grow with the basic row's, slot 2 m + 1: the z-reflected one
+struct ZItemDev {
+  int rec0, nrec;       // the path group's records (nrec a multiple of 4)
+  int flags;            // T: bit 0 swap x/y, bit 1 negate x, bit 2 negate y
+  int pad;
+  int16_t z0[8], z1[8];  // stored plane (z + 512) of each chain at the first column and at the end
+  int2 slot[2 * kZChains];         // (index into lines[], basic bin) or (-1, -1)
+  int16_t boff[2 * kZChains];      // back projection: the slot's datum 0 in the item's shared buffer (max_back floats)
+  int8_t owner[4 * ((2 * kZChains + 3) / 4)];  // the slot whose sums this one shares (two chains of one line)
+};
+
+struct ZParams {
+  const ZRec* recs;
+  const ZItemDev* items;
+  int nm;         // chains per item the kernels are compiled for: 4 or 6
+  int planes;     // planes per lane: 1, 2 or 4 (32 x planes >= nz)
+  int mean_rec;   // mean records of a path's groups
+  int max_out;    // most projection values of one item
+  int max_back;   // longest shared buffer of an item's data with the zeros around them
+};
+
+// Warps that share an item of a call with n items: a call with few items leaves most of the GPU's warps idle while each
+// walks hundreds of columns, so the CTA's four warps take a quarter of the path each.  A part repeats the item's set-up, so
+// calls that fill the forward kernel's 16 warps per SM, and short paths, keep a warp an item.  Measured, warp an item /
+// shared: 23 rings, 204 x 204 x 45, one of 21 subsets (OSEM step) 246 / 187 us; 12 rings, 290 x 290 x 23, one of 14
+// subsets (forward and back) 141 / 55 us; clinical, one of 21 subsets (4140 items, OSEM step) 752 / 860 us.
+constexpr int kZSplitItems = 2368, kZSplitRecords = 64;
+inline int z_parts(const ZParams& z, int n) { return n <= kZSplitItems && z.mean_rec >= kZSplitRecords ? kZWarps : 1; }
+
+// column stride (floats) of the padded images the kernels use when planes > 1
+inline int z_stride(const ZParams& z) { return 32 * z.planes; }
+
+// image [col][nz] <-> padded [col][stride] (planes past nz are zeros), `batch` images at the given strides
+cudaError_t launch_pad_image(const float* in, int64_t in_stride, float* out, int64_t out_stride, int64_t ncols, int nz,
+                             int stride, int batch, cudaStream_t st);
+cudaError_t launch_unpad_image(const float* in, int64_t in_stride, float* out, int64_t out_stride, int64_t ncols, int nz,
+                               int stride, int batch, cudaStream_t st);
+
+// padded != 0: image has column stride z_stride(z) (16-byte aligned), else nz
+cudaError_t launch_forward_z(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* image,
+                             int64_t img_stride, int padded, float* out, int64_t out_stride, int batch, cudaStream_t st,
+                             const FwdEpilogue* ep);
+cudaError_t launch_back_z(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* pd, int64_t pd_stride,
+                          float* image, int64_t img_stride, int padded, int batch, cudaStream_t st, int zero_ends);
+cudaError_t launch_back_z_fixed(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* pd,
+                                unsigned long long* acc, const double* scale, cudaStream_t st, int zero_ends);
+
+// batched reconstructions of frames whose geometries share a kernel variant (z: one of them): persistent CTAs over units
+// of kZWarps (frame, item) work items; smem: the largest z_batch_smem of the frames' geometries
+inline bool z_same_variant(const ZParams& a, const ZParams& b) {
+  return a.nm == b.nm && a.planes == b.planes;
+}
+constexpr int kZShared = 1 << 30;  // BatchItem::frame: the unit's entries are one item, shared by its warps
+int z_batch_smem(const ZParams& z, bool forward);
+int z_batch_max_ctas_per_sm(const ZParams& z, bool forward, int smem);
+cudaError_t launch_z_batch(const ZParams& z, bool forward, const ProjParams* geoms, const ZParams* zgeoms,
+                           const BatchFrameDev* frames, const BatchItem* items, int nunits, unsigned* counter, int smem,
+                           int grid, cudaStream_t st);
+
+}  // namespace b200

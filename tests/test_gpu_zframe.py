@@ -1,0 +1,114 @@
+"""z-frame projections (csrc/zframe.cu) against the oracle at the sizes where they can go wrong: planes at and beside the
+lanes' 32, 64 and 128, rows of several chains (two rays per bin, span 1, a truncated last segment), rectangular images,
+several axial samplings per plane; and infinite values."""
+import numpy as np
+import pytest
+
+from stir_b200 import _abi
+from stir_b200 import geometry as G
+
+pytestmark = pytest.mark.gpu
+
+
+def _geometry(rings, span, delta, dets=64, tang=21, nz=None, ny=23, nx=23, rays=1, planes_per_ring=2):
+    sc = G.Scanner(rings, dets, 100.0, 0.0, 4.0, float(np.float32(np.pi * 100.0 / dets)))
+    pdi = G.ProjDataInfoCTI(sc, span, delta, dets // 2, tang)
+    nz = nz or planes_per_ring * (rings - 1) + 1
+    img = G.ImageGeometry(nz, ny, nx, (4.0 / planes_per_ring, 4.1, 4.1))
+    return pdi, img, rays
+
+
+CASES = {
+    "one plane": _geometry(1, 1, 0),
+    "31 planes": _geometry(16, 3, 10),
+    "33 planes": _geometry(17, 3, 16),
+    "63 planes": _geometry(32, 11, 27),
+    "65 planes": _geometry(33, 11, 32),
+    "127 planes": _geometry(64, 11, 60, dets=32, tang=11, ny=11, nx=11),
+    "129 planes": _geometry(65, 11, 60, dets=32, tang=11, ny=11, nx=11),
+    "two rays": _geometry(12, 5, 11, rays=2),
+    "two rays, 63 planes": _geometry(32, 9, 31, rays=2),
+    "span 1": _geometry(9, 1, 8),
+    "span 1, one plane a ring": _geometry(9, 1, 8, planes_per_ring=1),
+    "span 1, 4 planes a ring": _geometry(9, 1, 5, planes_per_ring=4),
+    "truncated segment": _geometry(20, 5, 8),
+    "rectangular": _geometry(11, 3, 7, ny=19, nx=31),
+    "even image": _geometry(10, 7, 9, ny=24, nx=24, tang=24),
+}
+
+
+@pytest.fixture(scope="module", params=list(CASES), ids=list(CASES))
+def case(request, cuda_device):
+    from oracle.oracle import Oracle
+    from stir_b200.projectors import RayTracingProjector
+    pdi, img, rays = CASES[request.param]
+    proj = RayTracingProjector(pdi, img, num_tangential_LORs=rays, device=cuda_device)
+    return pdi, img, proj, Oracle(proj.geometry)
+
+
+def _bound(orc):
+    """Relative error of a float sum of n non-negative products, each side at most n roundings of 2^-24; n: the longest
+    row, and for a voxel the lines through it (fewer than 4 per view and ring pair at these sizes)."""
+    g = orc.geometry
+    n = 4 * max(g.nx, g.ny) * 3 + 4 * g.num_views * g.num_rings
+    return 2 * n * 2.0 ** -24
+
+
+@pytest.mark.parametrize("subset", [(0, 1), (1, 4)])
+def test_forward_and_back_match_oracle(case, subset):
+    import torch
+    pdi, img, proj, orc = case
+    x = np.random.default_rng(3).uniform(0.5, 1.5, img.shape).astype(np.float32)
+    xd = proj.image_to_device_layout(torch.from_numpy(x).cuda())
+    got = proj.projdata_from_device_layout(proj.forward_dev(xd, subset_num=subset[0], num_subsets=subset[1])).cpu().numpy()
+    ref = orc.forward(x, *subset)
+    assert np.all(np.abs(got - ref) <= _bound(orc) * np.abs(ref) + 1e-12)
+    y = np.random.default_rng(4).uniform(0.5, 1.5, proj.projdata_size).astype(np.float32)
+    yd = proj.projdata_to_device_layout(torch.from_numpy(y).cuda())
+    ref = orc.back(y, *subset)
+    for mode in (_abi.BACKPROJECT_ATOMIC, _abi.BACKPROJECT_DETERMINISTIC):
+        got = proj.image_from_device_layout(proj.back_dev(yd, subset_num=subset[0], num_subsets=subset[1],
+                                                          mode=mode)).cpu().numpy()
+        # fixed point: at most one unit of the grid (2^-40 of the largest sum and less) a line's part, within the slack
+        assert np.all(np.abs(got - ref) <= _bound(orc) * np.abs(ref) + 1e-6 * ref.max() * (mode != _abi.BACKPROJECT_ATOMIC))
+    assert proj.device_status() == 0
+
+
+def test_infinite_values_reach_their_rows_only(case):
+    """An infinite voxel makes the lines through it infinite and no others NaN; an infinite datum its row's voxels."""
+    import torch
+    pdi, img, proj, orc = case
+    x = np.random.default_rng(5).uniform(0.5, 1.5, img.shape).astype(np.float32)
+    x[img.nz // 2, img.ny // 2, img.nx // 2 + 2] = np.inf
+    xd = proj.image_to_device_layout(torch.from_numpy(x).cuda())
+    got = proj.projdata_from_device_layout(proj.forward_dev(xd)).cpu().numpy()
+    ref = orc.forward(x)
+    assert not np.isnan(got).any() and np.array_equal(np.isinf(got), np.isinf(ref))
+    y = np.random.default_rng(6).uniform(0.5, 1.5, proj.projdata_size).astype(np.float32)
+    y[proj.projdata_size // 3] = np.inf
+    yd = proj.projdata_to_device_layout(torch.from_numpy(y).cuda())
+    got = proj.image_from_device_layout(proj.back_dev(yd)).cpu().numpy()
+    ref = orc.back(y)
+    assert not np.isnan(got).any() and np.array_equal(np.isinf(got), np.isinf(ref))
+
+
+def test_calls_on_two_streams(cuda_device):
+    """Two streams project through one projector at once: every call has padded images of its own."""
+    import torch
+    from stir_b200.projectors import RayTracingProjector
+    pdi, img, _ = CASES["63 planes"]
+    proj = RayTracingProjector(pdi, img, device=cuda_device)
+    xs = [torch.rand(proj.device_image_shape, device="cuda", generator=torch.Generator("cuda").manual_seed(k))
+          for k in range(2)]
+    ref = [proj.forward_dev(x) for x in xs]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    outs = [[proj.empty_projdata() for _ in range(8)] for _ in range(2)]
+    torch.cuda.synchronize()
+    for r in range(8):
+        for k in range(2):
+            proj.forward_dev(xs[k], out=outs[k][r], stream=streams[k])
+    torch.cuda.synchronize()
+    for k in range(2):
+        for o in outs[k]:
+            assert torch.equal(o, ref[k])
