@@ -59,6 +59,7 @@ struct b200rt_batch {
   int family = B200RT_BATCH_KERNELS_PATHS;
   int max_f[5] = {0, 0, 0, 0, 0}, max_b[5] = {0, 0, 0, 0, 0};
   int num_tof = 1;
+  bool tof_lanes = false;  // the TOF family's kernels: every geometry's by timing-bin lanes (tof.cu), or the grouped ones
   DevBuf<b200::BatchFrameDev> d_frames;
   DevBuf<unsigned int> counters;  // work-queue heads of the forward and back launches
   bool ready = false;
@@ -129,12 +130,14 @@ void batch_finalize(b200rt_batch& b) {
   cudaStream_t st = b.capture_stream;
   b.d_geoms.upload(gp, st);
   bool paths = true, tof_grouped = true, packed = true, deterministic = false;
+  b.tof_lanes = !b.geoms.empty();
   b.num_tof = b.geoms.empty() ? 1 : b.geoms[0]->params.num_tof;
   for (auto* h : b.geoms) {
     paths = paths && h->use_paths;
     // one timing-bin count for the whole batch (the kernels' group size)
     tof_grouped = tof_grouped && h->params.tof_w != nullptr && h->params.num_tof == b.num_tof;
     packed = packed && h->params.max_nax <= b200::kPackedMaxNax;
+    b.tof_lanes = b.tof_lanes && b200::tof_lanes(h->params);
   }
   for (auto& fp : b.frames) deterministic = deterministic || fp->mode == B200RT_BACKPROJECT_DETERMINISTIC;
   if (deterministic && !paths) throw std::invalid_argument("deterministic batched frames need the column-staged kernels");
@@ -243,8 +246,10 @@ void batch_finalize(b200rt_batch& b) {
     b.max_b[B200RT_BATCH_KERNELS_PATHS] = fits ? most[1] : 0;
   }
   if (b.avail[B200RT_BATCH_KERNELS_TOF_GROUPED]) {
-    b.max_f[B200RT_BATCH_KERNELS_TOF_GROUPED] = b200::batch_tof_max_ctas_per_sm(b.num_tof, true);
-    b.max_b[B200RT_BATCH_KERNELS_TOF_GROUPED] = b200::batch_tof_max_ctas_per_sm(b.num_tof, false);
+    b.max_f[B200RT_BATCH_KERNELS_TOF_GROUPED] = b.tof_lanes ? b200::batch_tof_lanes_max_ctas_per_sm(b.num_tof, true)
+                                                            : b200::batch_tof_max_ctas_per_sm(b.num_tof, true);
+    b.max_b[B200RT_BATCH_KERNELS_TOF_GROUPED] = b.tof_lanes ? b200::batch_tof_lanes_max_ctas_per_sm(b.num_tof, false)
+                                                            : b200::batch_tof_max_ctas_per_sm(b.num_tof, false);
   }
   if (b.avail[B200RT_BATCH_KERNELS_PACKED]) {
     b.max_f[B200RT_BATCH_KERNELS_PACKED] = b200::batch_packed_max_ctas_per_sm(true);
@@ -436,6 +441,10 @@ cudaError_t batch_launch(b200rt_batch& b, int dir, int k, int order, const Batch
     }
     return cudaSuccess;
   }
+  if (b.family == B200RT_BATCH_KERNELS_TOF_GROUPED && b.tof_lanes)
+    return n > 0 ? b200::launch_batch_tof_lanes(dir == 0, b.d_geoms.p, b.num_tof, b.d_frames.p, items, n,
+                                                b.counters.p + dir, grid, st)
+                 : cudaSuccess;
   if (b.family == B200RT_BATCH_KERNELS_TOF_GROUPED)
     return dir == 0 ? b200::launch_forward_batch_tof(b.d_geoms.p, b.num_tof, b.d_frames.p, items, n, b.counters.p, grid,
                                                      st)

@@ -508,8 +508,10 @@ void setup_projector(b200rt_projector& h) {
       // keep the non-TOF rows (now in tof_rows) and the weights of every timing bin for the TOF-grouped kernels
       std::swap(h.tof_basic_rows.p, tof_rows.p);
       std::swap(h.tof_basic_rows.n, tof_rows.n);
-      h.tof_w.alloc(std::max<int64_t>(src, 1) * nt);
-      ck(launch_tof_weights(h.tof_basic_rows.p, d_jobs.p, njobs, tp, nt, h.tof_w.p, h.stream), "TOF weights");
+      const int ws = tof_weight_stride(nt);
+      h.tof_w.alloc(std::max<int64_t>(src, 1) * ws);
+      ck(cudaMemsetAsync(h.tof_w.p, 0, sizeof(float) * h.tof_w.n, h.stream), "memset");  // past the timing bins
+      ck(launch_tof_weights(h.tof_basic_rows.p, d_jobs.p, njobs, tp, ws, h.tof_w.p, h.stream), "TOF weights");
       std::vector<ProjBinDev> tb(nb);
       h.h_tof_basic_view.resize(nb);
       for (int b = 0; b < nb; ++b) {
@@ -590,6 +592,7 @@ void setup_projector(b200rt_projector& h) {
   p.max_row_len = max_len;
   p.tof_basic_rows = h.tof_basic_rows.p;
   p.tof_w = h.tof_w.p;
+  p.tof_ws = tof_weight_stride(g.num_tof());
   p.tof_basic = h.tof_basic.p;
   p.uniform_npa = g.npa(0);
   p.max_nax = 0;

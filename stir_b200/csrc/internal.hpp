@@ -86,11 +86,12 @@ struct ProjParams {
   const int* view_slot;
   int max_nax;      // most axial positions of any segment
   // TOF data by basic bin (the TOF-grouped packed kernels): the non-TOF basic rows, every element's weight for
-  // each timing bin ([element][timing bin], 0 where the TOF row has no element) and one entry per basic bin
+  // each timing bin ([element][tof_ws], 0 where the TOF row has no element and past the timing bins) and one entry per basic bin
   // (row_offset into tof_basic_rows, tof = min timing bin); null without TOF
   const RowElem* tof_basic_rows;
   const float* tof_w;
   const ProjBinDev* tof_basic;
+  int tof_ws;       // floats of an element in tof_w: the timing bins in whole 16-byte pieces
 };
 // with at most this many axial positions per line the per-basic-bin kernels pack (line, axial position) pairs
 // into the lanes of a warp (project.cu)
@@ -488,8 +489,25 @@ struct TofParams {
   int erf_n;
   double erf_max, erf_period;
 };
-cudaError_t launch_tof_weights(const RowElem* src, const TofJobDev* jobs, int njobs, const TofParams& tp, int ntof,
+cudaError_t launch_tof_weights(const RowElem* src, const TofJobDev* jobs, int njobs, const TofParams& tp, int ws,
                                float* w, cudaStream_t st);
+// TOF projections with the timing bins over the lanes (tof.cu), where tof_lanes() holds
+int tof_weight_stride(int num_tof);
+// timing bins per pass of the TOF-grouped kernels: the fewest passes of at most 32 bins, spread evenly, rounded up to an
+// instantiated size
+__host__ __device__ inline int tof_group_size(int K) {
+  const int passes = (K + 31) / 32;
+  const int per = (K + passes - 1) / passes;
+  return per <= 8 ? 8 : per <= 16 ? 16 : per <= 20 ? 20 : per <= 24 ? 24 : 32;
+}
+bool tof_lanes(const ProjParams& p);
+cudaError_t launch_forward_tof_lanes(const ProjParams& p, const int* items, int nitems, const float* image, float* projdata,
+                                     cudaStream_t st, const FwdEpilogue& ep);
+cudaError_t launch_back_tof_lanes(const ProjParams& p, const int* items, int nitems, const float* projdata, float* image,
+                                  unsigned long long* acc, const double* scale, cudaStream_t st, int zero_ends);
+cudaError_t launch_batch_tof_lanes(bool forward, const ProjParams* geoms, int num_tof, const BatchFrameDev* frames,
+                                   const BatchItem* items, int nitems, unsigned* counter, int grid, cudaStream_t st);
+int batch_tof_lanes_max_ctas_per_sm(int num_tof, bool forward);
 // TOF-grouped packed projections over basic bins (items index ProjParams::tof_basic); forward with every epilogue
 // (kEpiLoglik: one partial per item); back atomic (float) or fixed point
 cudaError_t launch_forward_tof_grouped(const ProjParams& p, const int* items, int nitems, const float* image,

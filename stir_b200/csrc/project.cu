@@ -633,7 +633,7 @@ size_t proj_smem_bytes(int max_row_len) {
 // one atomic (float), or, in fixed point, summed in float in that fixed order and rounded once to an integer.
 constexpr int kTofWarps = 4;
 constexpr int kTofMinCtas = 8;  // 64 registers: 32 warps per SM (79 registers left 24)
-constexpr int kTofGroupMax = 32;  // timing bins per pass: KG in {8, 16, 20, 24, 32}, chosen from their number
+// timing bins per pass: KG in {8, 16, 20, 24, 32}, chosen from their number (tof_group_size)
 template <int KG>
 struct TofStage {
   int2 xs[kPackedMaxLines][33];
@@ -644,7 +644,7 @@ struct TofStage {
 // timing bins [k0, k0 + KG)
 template <int KG>
 __device__ __forceinline__ void tof_stage_batch(const ProjParams& p, const ProjBinDev& pb, const RowElem* row,
-                                                const float* wrow, int K, int l0, int ng, int e0, int cnt, int k0,
+                                                const float* wrow, int K, int ws, int l0, int ng, int e0, int cnt, int k0,
                                                 TofStage<KG>& S, int lane) {
   __syncwarp();
   if (lane < cnt) {
@@ -660,12 +660,12 @@ __device__ __forceinline__ void tof_stage_batch(const ProjParams& p, const ProjB
       S.xs[g][lane] = make_int2(((yt - p.min_y) * p.nx + (xt - p.min_x)) * p.nz, zt);
     }
   }
-  // weights: the batch's elements x timing bins are contiguous ([element][timing bin]); coalesced loads
+  // weights: the batch's elements are contiguous ([element][ws]); coalesced loads
   float* sw = reinterpret_cast<float*>(S.w);
-  const float* src = wrow + static_cast<int64_t>(e0) * K;
+  const float* src = wrow + static_cast<int64_t>(e0) * ws;
   for (int i = lane; i < 32 * KG; i += 32) {
     const int e = i / KG, kk = i % KG;
-    sw[e * KG + kk] = (e < cnt && k0 + kk < K) ? __ldg(src + static_cast<int64_t>(e) * K + k0 + kk) : 0.f;
+    sw[e * KG + kk] = (e < cnt && k0 + kk < K) ? __ldg(src + static_cast<int64_t>(e) * ws + k0 + kk) : 0.f;
   }
   __syncwarp();
 }
@@ -677,7 +677,7 @@ __device__ __forceinline__ void forward_tof_grouped_body(const ProjParams& p, co
                                                          int lane) {
   const RowElem* row = p.tof_basic_rows + pb.row_offset;
   const int K = p.num_tof;
-  const float* wrow = p.tof_w + pb.row_offset * K;
+  const float* wrow = p.tof_w + pb.row_offset * p.tof_ws;
   const int nax = packed_nax(p, pb);
   const bool blocked = nax > kPackedMaxNax;
   const int G = blocked ? 1 : min(32 / nax, kPackedMaxLines);
@@ -693,7 +693,7 @@ __device__ __forceinline__ void forward_tof_grouped_body(const ProjParams& p, co
       for (int kk = 0; kk < KG; ++kk) acc[kk] = 0.f;
       for (int e0 = 0; e0 < pb.row_len; e0 += 32) {
         const int cnt = min(32, pb.row_len - e0);
-        tof_stage_batch<KG>(p, pb, row, wrow, K, l0, ng, e0, cnt, k0, S, lane);
+        tof_stage_batch<KG>(p, pb, row, wrow, K, p.tof_ws, l0, ng, e0, cnt, k0, S, lane);
         if (t.act)
           for (int k = 0; k < cnt; ++k) {
             const int2 X = S.xs[gi][k];
@@ -771,7 +771,7 @@ __device__ __forceinline__ void back_tof_grouped_body(const ProjParams& p, const
                                                       int lane) {
   const RowElem* row = p.tof_basic_rows + pb.row_offset;
   const int K = p.num_tof;
-  const float* wrow = p.tof_w + pb.row_offset * K;
+  const float* wrow = p.tof_w + pb.row_offset * p.tof_ws;
   const int nax = packed_nax(p, pb);
   const bool blocked = nax > kPackedMaxNax;
   const int G = blocked ? 1 : min(32 / nax, kPackedMaxLines);
@@ -795,7 +795,7 @@ __device__ __forceinline__ void back_tof_grouped_body(const ProjParams& p, const
       if (!__any_sync(0xffffffffu, any)) continue;
       for (int e0 = 0; e0 < pb.row_len; e0 += 32) {
         const int cnt = min(32, pb.row_len - e0);
-        tof_stage_batch<KG>(p, pb, row, wrow, K, l0, ng, e0, cnt, k0, S, lane);
+        tof_stage_batch<KG>(p, pb, row, wrow, K, p.tof_ws, l0, ng, e0, cnt, k0, S, lane);
         if (any)
           for (int k = 0; k < cnt; ++k) {
             const int2 X = S.xs[gi][k];
@@ -1053,13 +1053,6 @@ int batch_packed_max_ctas_per_sm(bool forward) {
   return n;
 }
 
-// timing bins per pass: the fewest passes of at most 32 bins, spread evenly, rounded up to an instantiated size
-int tof_group_size(int K) {
-  const int passes = (K + kTofGroupMax - 1) / kTofGroupMax;
-  const int per = (K + passes - 1) / passes;
-  return per <= 8 ? 8 : per <= 16 ? 16 : per <= 20 ? 20 : per <= 24 ? 24 : 32;
-}
-
 #define TOF_KG_SWITCH(K, CALL)                       \
   switch (tof_group_size(K)) {                       \
     case 8: { constexpr int KG = 8; CALL; break; }   \
@@ -1074,6 +1067,7 @@ cudaError_t launch_forward_tof_grouped(const ProjParams& p, const int* items, in
   if (nitems <= 0) return cudaSuccess;
   const int grid = (nitems + kTofWarps - 1) / kTofWarps;
   FwdEpilogue none{};
+  if (tof_lanes(p)) return launch_forward_tof_lanes(p, items, nitems, image, projdata, st, ep ? *ep : none);
   if (!ep || ep->mode == kEpiNone) {
     TOF_KG_SWITCH(p.num_tof, (forward_tof_grouped_kernel<KG, kEpiNone><<<grid, kTofWarps * 32, 0, st>>>(
                                  p, items, nitems, image, projdata, none)));
@@ -1094,6 +1088,7 @@ cudaError_t launch_back_tof_grouped(const ProjParams& p, const int* items, int n
                                     float* image, unsigned long long* acc, const double* scale, cudaStream_t st,
                                     int zero_ends) {
   if (nitems <= 0) return cudaSuccess;
+  if (tof_lanes(p)) return launch_back_tof_lanes(p, items, nitems, projdata, image, acc, scale, st, zero_ends);
   const int grid = (nitems + kTofWarps - 1) / kTofWarps;
   if (acc) {
     TOF_KG_SWITCH(p.num_tof, (back_tof_grouped_kernel<KG, TofFixedSum><<<grid, kTofWarps * 32, 0, st>>>(

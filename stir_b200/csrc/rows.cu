@@ -349,7 +349,7 @@ __global__ void tof_rows_kernel(const RowElem* __restrict__ src, const TofJobDev
 // w[(src_offset + e) * ntof + tof_index] = the TOF row's value (e.v * kernel value), 0 where the TOF row has no
 // element (the same arithmetic as tof_rows_kernel, so the weights equal the TOF rows' values)
 __global__ void tof_weights_kernel(const RowElem* __restrict__ src, const TofJobDev* __restrict__ jobs, int njobs,
-                                   TofParams tp, int ntof, float* __restrict__ w) {
+                                   TofParams tp, int ws, float* __restrict__ w) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= njobs) return;
   const TofJobDev job = jobs[j];
@@ -367,16 +367,16 @@ __global__ void tof_weights_kernel(const RowElem* __restrict__ src, const TofJob
     ip = ip + (px - job.mid[2]) * job.unit[2];
     const float d2 = -ip;
     const float kv = tof_value(tp, low - d2, high - d2);
-    w[(job.src_offset + k) * ntof + job.tof_index] = (kv > 0 && e.v != 0) ? e.v * kv : 0.f;
+    w[(job.src_offset + k) * ws + job.tof_index] = (kv > 0 && e.v != 0) ? e.v * kv : 0.f;
   }
 }
 
 }  // namespace
 
-cudaError_t launch_tof_weights(const RowElem* src, const TofJobDev* jobs, int njobs, const TofParams& tp, int ntof,
+cudaError_t launch_tof_weights(const RowElem* src, const TofJobDev* jobs, int njobs, const TofParams& tp, int ws,
                                float* w, cudaStream_t st) {
   if (njobs <= 0) return cudaSuccess;
-  tof_weights_kernel<<<(njobs + 127) / 128, 128, 0, st>>>(src, jobs, njobs, tp, ntof, w);
+  tof_weights_kernel<<<(njobs + 127) / 128, 128, 0, st>>>(src, jobs, njobs, tp, ws, w);
   return cudaGetLastError();
 }
 
