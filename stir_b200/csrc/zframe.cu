@@ -583,13 +583,17 @@ __global__ void __launch_bounds__(kZWarps * 32, forward_ctas(NM, P))
 
 // What becomes of a column's sums u (planes lane + 32 j): floats added to the padded or the plain image, or rounded once
 // per item to the fixed-point grid (a power-of-two scale: exact) and added as 64-bit integers, in any order the same sum.
+// PAD: the columns hold every plane of the lanes, so none has to be left out.
+template <bool PAD>
 struct ZFloatSink {
+  static constexpr bool kWhole = PAD;
   float* img;
   __device__ __forceinline__ void load() {}
   __device__ __forceinline__ void batch(int64_t o) { img += o; }
   __device__ __forceinline__ void add(int i, float v) const { atomicAdd(img + i, v); }
 };
 struct ZFixedSink {
+  static constexpr bool kWhole = false;
   unsigned long long* acc;
   const double* scale_ptr;
   float scale;
@@ -751,7 +755,7 @@ __device__ __forceinline__ void back_z_item(const ProjParams& p, const ZParams& 
       const int i = offs[k] + lane;
 #pragma unroll
       for (int j = 0; j < P; ++j)
-        if (lane + 32 * j < p.nz) sink.add(i + 32 * j, v[j]);
+        if (Sink::kWhole || lane + 32 * j < p.nz) sink.add(i + 32 * j, v[j]);
     }
   }
   cp_wait<0>();
@@ -834,7 +838,7 @@ __global__ void __launch_bounds__(kZWarps * 32, back_ctas(P))
       back_z_item<NM, P>(p, z, z.items[wi.bin], ring, part, parts, f.ratio, sink, p.nz, 0, lane);
     } else {
       constexpr bool kPad = P > 1;
-      const ZFloatSink sink{kPad ? f.upad : f.u};
+      const ZFloatSink<kPad> sink{kPad ? f.upad : f.u};
       back_z_item<NM, P>(p, z, z.items[wi.bin], ring, part, parts, f.ratio, sink, kPad ? 32 * P : p.nz, 0, lane);
     }
   }
@@ -948,8 +952,14 @@ cudaError_t launch_back_z(const ProjParams& p, const ZParams& z, const int* list
                           int64_t pd_stride,
                           float* image, int64_t img_stride, int padded, int batch, cudaStream_t st, int zero_ends) {
   return z_variant(z, [&]<int NM, int P>() {
-    return launch_z(back_z_kernel<NM, P, ZFloatSink>, kZWarps * z_warp_smem(z, false), n, parts, batch, st, p, z, list, n, parts, pd,
-                    pd_stride, ZFloatSink{image}, img_stride, padded ? z_stride(z) : p.nz, zero_ends);
+    const int sm = kZWarps * z_warp_smem(z, false);
+    if constexpr (P > 1) {
+      if (padded)
+        return launch_z(back_z_kernel<NM, P, ZFloatSink<true>>, sm, n, parts, batch, st, p, z, list, n, parts, pd, pd_stride,
+                        ZFloatSink<true>{image}, img_stride, z_stride(z), zero_ends);
+    }
+    return launch_z(back_z_kernel<NM, P, ZFloatSink<false>>, sm, n, parts, batch, st, p, z, list, n, parts, pd, pd_stride,
+                    ZFloatSink<false>{image}, img_stride, p.nz, zero_ends);
   });
 }
 
