@@ -31,8 +31,8 @@ WORKLOAD = ("clinical 3D PET: 64 rings x 504 det, R 328 mm, span 11, max ring di
             "(72,557,856 LORs), image 344x344x127 (2.09x2.09x2.03 mm), ray-tracing matrix, 1 tangential LOR")
 METRIC = "fwd+back LORs/s"
 CPU_SAMPLE_SUBSET = (0, 42)  # views 0, 42 and their symmetry partners: 1/42 of the views
-# the column-staged projectors (stir_b200/csrc/paths.cu) that project the clinical workload
-FWD_KERNEL, BACK_KERNEL = "forward_paths_kernel", "back_paths_kernel"
+# the z-frame projectors (stir_b200/csrc/zframe.cu) that project the clinical workload
+FWD_KERNEL, BACK_KERNEL = "forward_z_kernel", "back_z_kernel"
 
 
 def parse():
@@ -440,7 +440,7 @@ def tof_workload(with_cpu, device):
         res = {"metric": "TOF fwd+back TOF-bin LORs/s", "value": n / ((fms + bms) / 1e3), "unit": "LORs/s",
                "tof_bins_per_step": n, "forward_ms": fms, "back_ms": bms, "setup_s": setup_s, "gpu_launches": 2,
                "workload": "8 rings x 288 det (R 300 mm), span 1, 144 views x 64 tang, 33 timing bins of 50 ps, "
-                           "Gaussian 550 ps FWHM (STIR's kernel cut-off), image 64x64x15; TOF-grouped kernels",
+                           "Gaussian 550 ps FWHM (STIR's kernel cut-off), image 64x64x15; timing-bin lanes",
                "row_elements": int(proj.info.total_nnz)}
         # the same with the Gaussian truncated at +-3 sigma (the kernel of the TOF configuration) beside STIR's cut-off
         p3 = RayTracingProjector(pdi, img, device=device, tof_kernel_truncation_sigmas=3.0)
@@ -833,8 +833,8 @@ def b200_main(args):
                             BACK_KERNEL: profile_value("l2_hit_rate", BACK_KERNEL)}}
 
     roof["byte_model"] = ("algorithmic bytes: every (row element, LOR) pair counted as a 4-byte image read "
-                          "(forward) or an 8-byte read-modify-write (back); the column staging serves them from shared "
-                          "memory and L2, so frac above 1 says the kernel avoids DRAM, not that it beats the copy "
+                          "(forward) or an 8-byte read-modify-write (back); the kernels serve them from registers, "
+                          "shared memory and L2, so frac above 1 says the kernel avoids DRAM, not that it beats the copy "
                           "bandwidth; the compulsory-bytes fractions (image and projection data once) and the on-chip "
                           "limiter (ncu) say where the time goes")
 
