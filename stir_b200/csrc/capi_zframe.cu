@@ -1,32 +1,8 @@
 // Set-up of the z-frame tables and the dispatch between the two path-item projections (z-frame, column-staged).
 #include "capi.hpp"
+#include "zchains.hpp"
 
 using namespace b200;
-
-namespace {
-
-// a chain of one member: per column its element before the event (w1), whether it moves up there, and the element after
-struct Chain {
-  int member;
-  int cur, z0;  // stored plane (z + 512) now and at the first column
-};
-
-struct Group {
-  std::vector<std::vector<ZRec>> recs;               // per chain group
-  std::vector<std::vector<int>> chain_member;        // per chain group: the member of every chain
-  std::vector<std::vector<int>> chain_z0, chain_z1;  // planes (z + 512) at the first column and at the end
-  bool ok = true;
-};
-
-// An event from stored plane zr to zr + 1 of a line (zt: plane of axial position 0 before it; dz: its move, 1 or -1):
-// the axial position that leaves the planes [0, planes), or -1, and whether one enters
-void edge_event(int zt, int dz, int nax, int npa, int planes, int& leave, bool& enters) {
-  auto at = [&](int d) { return d >= 0 && d % npa == 0 && d / npa < nax ? d / npa : -1; };
-  leave = dz > 0 ? at(planes - 1 - zt) : at(-zt);
-  enters = (dz > 0 ? at(-(zt + 1)) : at(planes - 1 - (zt - 1))) >= 0;
-}
-
-}  // namespace
 
 namespace capi {
 
@@ -44,180 +20,31 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   if (padded >= (int64_t(1) << 31)) return false;
   const int ngroups = nviews * ntangs;
   const int planes = 32 * z.planes;
-
-  struct Elem {
-    int z;
-    float v;
-  };
+  ZPathLines fit;
+  fit.S = g.S();
+  fit.min_z = p.min_z;
+  fit.planes = planes;
+  for (int sg = -g.S(); sg <= g.S(); ++sg) {
+    fit.nax.push_back(g.nax(sg));
+    fit.npa.push_back(g.npa(sg));
+  }
   // pass 0 counts the chains a path needs, pass 1 builds the records for groups of z.nm chains
-  std::vector<Group> groups(ngroups);
+  std::vector<ZPath> groups(ngroups);
   std::vector<int> chains_of(ngroups, 0), chains_max(ngroups, 0);
-  auto work = [&](int g0, int g1, int cap) {
-    std::vector<uint32_t> keys;
-    std::vector<int> order;
-    for (int gi = g0; gi < g1; ++gi) {
-      Group& G = groups[gi];
-      try {
-        const int vi = gi / ntangs, ti = gi % ntangs;
-        keys.clear();
-        for (int si = 0; si < nsegs; ++si) {
-          const ProjBinDev& pb = h.h_bins[(static_cast<size_t>(vi) * nsegs + si) * ntangs + ti];
-          for (int k = 0; k < pb.row_len; ++k) keys.push_back(hr[pb.row_offset + k].zyx & 0x3fffffu);  // x, y bits
-        }
-        std::sort(keys.begin(), keys.end());
-        keys.erase(std::unique(keys.begin(), keys.end()), keys.end());
-        const int ncols = static_cast<int>(keys.size());
-        // every member's elements by column, planes ascending within a column
-        std::vector<std::vector<std::vector<Elem>>> el(nsegs, std::vector<std::vector<Elem>>(ncols));
-        for (int si = 0; si < nsegs; ++si) {
-          const ProjBinDev& pb = h.h_bins[(static_cast<size_t>(vi) * nsegs + si) * ntangs + ti];
-          for (int k = 0; k < pb.row_len; ++k) {
-            const RowElem e = hr[pb.row_offset + k];
-            const size_t c = std::lower_bound(keys.begin(), keys.end(), e.zyx & 0x3fffffu) - keys.begin();
-            el[si][c].push_back(Elem{static_cast<int>(e.zyx >> 22), e.v});
-          }
-          for (auto& v : el[si])
-            std::stable_sort(v.begin(), v.end(), [](const Elem& a, const Elem& b) { return a.z < b.z; });
-        }
-        // the columns along the path: a ray steps in x or in y, so x + y (or x - y) orders them; away from the end where
-        // the steepest member's planes are higher
-        double mx = 0, my = 0, cov = 0;
-        for (uint32_t k : keys) mx += k & 2047u, my += k >> 11;
-        mx /= ncols, my /= ncols;
-        for (uint32_t k : keys) cov += ((k & 2047u) - mx) * ((k >> 11) - my);
-        const int sy = cov >= 0 ? 1 : -1;
-        auto along = [&](int c) { return static_cast<int>(keys[c] & 2047u) + sy * static_cast<int>(keys[c] >> 11); };
-        order.resize(ncols);
-        for (int c = 0; c < ncols; ++c) order[c] = c;
-        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return along(a) < along(b); });
-        {
-          double s0 = 0, s1 = 0, n0 = 0, n1 = 0;  // mean plane of the last member in the two halves
-          for (int i = 0; i < ncols; ++i)
-            for (const Elem& e : el[nsegs - 1][order[i]]) (i < ncols / 2 ? s0 : s1) += e.z, (i < ncols / 2 ? n0 : n1) += 1;
-          if (n0 > 0 && n1 > 0 && s0 / n0 > s1 / n1) std::reverse(order.begin(), order.end());
-        }
-        // chains: each element goes to the member's chain with the highest plane not above it (one element per plane)
-        struct Link {
-          int chain;
-          Elem e;
-        };
-        std::vector<std::vector<Chain>> chains(nsegs);
-        std::vector<std::vector<std::vector<Link>>> links(nsegs, std::vector<std::vector<Link>>(ncols));
-        int total = 0, most = 0;
-        for (int si = 0; si < nsegs; ++si) {
-          for (int i = 0; i < ncols; ++i)
-            for (const Elem& e : el[si][order[i]]) {
-              int best = -1;
-              for (int c = 0; c < static_cast<int>(chains[si].size()); ++c) {
-                const int cz = chains[si][c].cur;
-                // a chain that is at this plane already in this column has taken the element of a merged ray
-                if (cz <= e.z && (best < 0 || cz > chains[si][best].cur)) best = c;
-              }
-              if (best < 0) {
-                best = static_cast<int>(chains[si].size());
-                chains[si].push_back(Chain{si, e.z, e.z});
-              }
-              chains[si][best].cur = e.z;
-              links[si][i].push_back(Link{best, e});
-            }
-          // lines of an empty row are projected too (to 0): a chain without elements
-          if (chains[si].empty()) chains[si].push_back(Chain{si, 512, 512});
-          total += static_cast<int>(chains[si].size());
-          most = std::max(most, static_cast<int>(chains[si].size()));
-        }
-        chains_of[gi] = total;
-        chains_max[gi] = most;
-        if (cap == 0) continue;
-        // members into groups of at most cap chains, in order
-        std::vector<std::vector<int>> members;
-        int fill = cap + 1;
-        for (int si = 0; si < nsegs; ++si) {
-          const int n = static_cast<int>(chains[si].size());
-          if (fill + n > cap) {
-            members.emplace_back();
-            fill = 0;
-          }
-          members.back().push_back(si);
-          fill += n;
-        }
-        for (const auto& mem : members) {
-          std::vector<int> cm, cz0, first(nsegs, 0);
-          for (int si : mem) {
-            first[si] = static_cast<int>(cm.size());
-            for (const Chain& c : chains[si]) {
-              cm.push_back(si);
-              cz0.push_back(c.z0);
-            }
-          }
-          const int nc = static_cast<int>(cm.size());
-          std::vector<int> cur = cz0;
-          std::vector<ZRec> recs;
-          for (int i = 0; i < ncols; ++i) {
-            const size_t head = recs.size();
-            auto fresh = [&]() {
-              ZRec r{};
-              r.xy = keys[order[i]];
-              recs.push_back(r);
-            };
-            fresh();
-            for (int si : mem)
-              for (const Link& l : links[si][i]) {
-                const int m = first[si] + l.chain;
-                // up to the element's plane: one event a record, in further records of the column where one is not enough
-                size_t k = head;
-                while (cur[m] < l.e.z) {
-                  while (k < recs.size() && (recs[k].op & (1u << m))) ++k;
-                  if (k == recs.size()) fresh();
-                  recs[k].op |= 1u << m;
-                  // what leaves and enters: the same for every line of the member in one z orientation (checked)
-                  const ProjBinDev& pb = h.h_bins[(static_cast<size_t>(vi) * nsegs + si) * ntangs + ti];
-                  int leave[2] = {-2, -2};
-                  for (int q = 0; q < pb.num_lines; ++q) {
-                    const LineDev& L = lines[pb.first_line + q];
-                    const int d = (L.flags & 8) ? 1 : 0;
-                    const int zt = d ? L.q + 512 - p.min_z - cur[m] : cur[m] - 512 - p.min_z;
-                    int out = -1;
-                    bool in = false;
-                    edge_event(zt, d ? -1 : 1, g.nax(L.seg), g.npa(L.seg), planes, out, in);
-                    if (leave[d] != -2 && leave[d] != out) G.ok = false;
-                    leave[d] = out;
-                    if (out >= 0 || in) recs[k].op |= 1u << (6 + m);
-                  }
-                  recs[k].leave[m] = static_cast<int32_t>((static_cast<uint32_t>(std::max(leave[1], -1)) << 16) |
-                                                          (static_cast<uint32_t>(std::max(leave[0], -1)) & 0xffffu));
-                  ++cur[m];
-                }
-                // the element: before the column's events at the chain's first plane here, after the event otherwise
-                bool placed = false;
-                for (size_t q = recs.size(); q-- > head;)
-                  if (recs[q].op & (1u << m)) {
-                    recs[q].w2[m] += l.e.v;
-                    placed = true;
-                    break;
-                  }
-                if (!placed) recs[head].w1[2 * m] += l.e.v;
-              }
-          }
-          while (recs.size() % 4) {  // the kernels take four records at a time
-            ZRec r{};
-            r.xy = recs.back().xy;
-            recs.push_back(r);
-          }
-          for (ZRec& r : recs) {
-            for (int m = 0; m < nc; ++m) {
-              if (r.w1[2 * m] == 0.f) r.op |= kZGuard;
-              r.w1[2 * m + 1] = r.w1[2 * m];
-              if ((r.op >> m & 1u) && r.w2[m] == 0.f) r.op |= 1u << (6 + m);
-            }
-          }
-          G.recs.push_back(std::move(recs));
-          G.chain_member.push_back(std::move(cm));
-          G.chain_z0.push_back(std::move(cz0));
-          G.chain_z1.push_back(std::move(cur));
-        }
-      } catch (const std::exception&) {
-        G.ok = false;
+  auto work = [&](int gi, int cap) {
+    ZPath& G = groups[gi];
+    try {
+      const int vi = gi / ntangs, ti = gi % ntangs;
+      std::vector<ZMember> members(nsegs);
+      for (int si = 0; si < nsegs; ++si) {
+        const ProjBinDev& pb = h.h_bins[(static_cast<size_t>(vi) * nsegs + si) * ntangs + ti];
+        members[si] = ZMember{hr.data() + pb.row_offset, pb.row_len, lines.data() + pb.first_line, pb.num_lines};
       }
+      build_path(members, fit, cap, G);
+      chains_of[gi] = G.total;
+      chains_max[gi] = G.most;
+    } catch (const std::exception&) {
+      G.ok = false;
     }
   };
   const int nthreads = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
@@ -226,7 +53,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
     for (int t = 0; t < nthreads; ++t)
       pool.emplace_back([&, t] {
         // interleaved: neighbouring paths cost about the same
-        for (int gi = t * stride; gi < ngroups; gi += nthreads * stride) work(gi, gi + 1, cap);
+        for (int gi = t * stride; gi < ngroups; gi += nthreads * stride) work(gi, cap);
       });
     for (auto& th : pool) th.join();
   };
@@ -248,7 +75,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   if (most > kZChains) return false;
   if (most > z.nm) {  // a path outside the sample needs more
     z.nm = kZChains;
-    for (Group& G : groups) G = Group{};
+    for (ZPath& G : groups) G = ZPath{};
     run(1, z.nm);
   }
   int64_t nrecs = 0;
@@ -281,7 +108,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
         for (int ti = t0; ti < t1; ++ti) most_groups = std::max(most_groups, groups[vi * ntangs + ti].recs.size());
         for (size_t gr = 0; gr < most_groups; ++gr)
           for (int ti = t0; ti < t1; ++ti) {
-            const Group& G = groups[vi * ntangs + ti];
+            const ZPath& G = groups[vi * ntangs + ti];
             if (gr >= G.recs.size()) continue;
             int rec0 = base[vi * ntangs + ti];
             for (size_t k = 0; k < gr; ++k) rec0 += static_cast<int>(G.recs[k].size());
@@ -402,7 +229,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   ck(cudaMemsetAsync(h.dev_status.p, 0, sizeof(unsigned), h.stream), "memset");
   ck(cudaStreamSynchronize(h.stream), "path tables");
   int64_t ngrp = 0;
-  for (const Group& G : groups) ngrp += static_cast<int64_t>(G.recs.size());
+  for (const ZPath& G : groups) ngrp += static_cast<int64_t>(G.recs.size());
   z.mean_rec = static_cast<int>(nrecs / std::max<int64_t>(1, ngrp));
   z.recs = h.z_recs.p;
   z.items = h.z_items.p;
