@@ -143,6 +143,7 @@ struct b200rt_projector {
   bool use_z = false;
   DevBuf<ZRec> z_recs;
   DevBuf<ZItemDev> z_items;
+  DevBuf<ZPlanes> z_planes;
   ZParams zparams{};
   cudaMemPool_t z_pool = nullptr;  // padded images of calls in flight
   std::vector<char> h_item_lead;   // the first of a path item's parts (groups of chains, further lines)
@@ -203,6 +204,9 @@ void forward_subset(b200rt_projector& h, const float* image, float* out, int sub
                     const FwdEpilogue* ep = nullptr);
 bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std::vector<LineDev>& lines, int nviews,
                   int nsegs, int ntangs, const std::vector<int>& bviews);
+// how a call's n items are walked (zframe.hpp)
+ZSplit z_split(const b200rt_projector& h, int n);
+int z_back_parts(const b200rt_projector& h, int n);
 // path-item projections of a list of items for a batch of images (use_paths).  n_call: the items of the whole call where
 // the list is a part of it (-1: the list is)
 void forward_paths(b200rt_projector& h, const int* list, int n, const float* images, int64_t img_stride, float* out,

@@ -314,16 +314,22 @@ const BatchItem* batch_items(b200rt_batch& b, int k, int order, int& count) {
     per_frame[fi] = std::move(bins);
   }
   // the frame's entries of the list, in units of `unit` that stay together: z-frame kernels take kZWarps items a CTA, or
-  // one item kZWarps times where the frame's own call would share it between the warps (z_parts)
+  // items repeated for each warp that shares one, walked as in the frame's own call (z_split)
   std::vector<std::vector<BatchItem>> entries(b.frames.size());
   std::vector<size_t> unit(b.frames.size(), 1);
   for (size_t fi = 0; fi < b.frames.size(); ++fi) {
     const b200rt_projector& h = *b.frames[fi]->h;
     const int frame = static_cast<int>(fi);
     const bool zf = b.family == B200RT_BATCH_KERNELS_PATHS && h.use_z;
-    const int parts = zf ? b200::z_parts(h.zparams, static_cast<int>(per_frame[fi].size())) : 1;
+    int parts = 1, code = frame;
+    if (zf) {
+      if (frame >> b200::kZFrameBits) throw std::invalid_argument("too many batched frames");
+      b200::ZSplit sp = z_split(h, static_cast<int>(per_frame[fi].size()));
+      parts = sp.parts = std::min(sp.parts, b200::kZWarps);
+      code = b200::z_frame_split(frame, sp);
+    }
     for (int bin : per_frame[fi])
-      for (int q = 0; q < parts; ++q) entries[fi].push_back(BatchItem{frame | (parts > 1 ? b200::kZShared : 0), bin});
+      for (int q = 0; q < parts; ++q) entries[fi].push_back(BatchItem{code, bin});
     if (zf) {
       unit[fi] = b200::kZWarps;
       while (entries[fi].size() % b200::kZWarps) entries[fi].push_back(BatchItem{frame, -1});
@@ -355,7 +361,7 @@ const BatchItem* batch_items(b200rt_batch& b, int k, int order, int& count) {
     for (size_t k = 0; k < b.path_kernels.size(); ++k) {
       const int first = static_cast<int>(by.size());
       for (const BatchItem& it : list)
-        if (b.geom_kernel[b.frames[it.frame & ~b200::kZShared]->geom] == static_cast<int>(k)) by.push_back(it);
+        if (b.geom_kernel[b.frames[it.frame & ((1 << b200::kZFrameBits) - 1)]->geom] == static_cast<int>(k)) by.push_back(it);
       parts.push_back({static_cast<int>(k), first, static_cast<int>(by.size()) - first});
     }
     list.swap(by);

@@ -992,6 +992,7 @@ void b200rt_destroy(b200rt_projector* h) {
     h->ossps_minpos.release();
     h->z_recs.release();
     h->z_items.release();
+    h->z_planes.release();
     h->z_work.release();
     h->z_partials.release();
     h->path_elems.release();

@@ -90,9 +90,12 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   std::vector<char> item_lead;  // the first item of a (path, T)
   std::vector<PathItemDev> path_items;
   std::vector<char> led(static_cast<size_t>(ntangs));
-  std::vector<int> base(ngroups);
+  std::vector<int> base(ngroups), path0(ngroups);
+  std::vector<ZPlanes> sixteenths;
   int64_t at = 0;
   for (int gi = 0; gi < ngroups; ++gi) {
+    path0[gi] = static_cast<int>(sixteenths.size());
+    sixteenths.insert(sixteenths.end(), groups[gi].planes.begin(), groups[gi].planes.end());
     base[gi] = static_cast<int>(at);
     for (const auto& r : groups[gi].recs) at += static_cast<int64_t>(r.size());
   }
@@ -113,20 +116,20 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
             int rec0 = base[vi * ntangs + ti];
             for (size_t k = 0; k < gr; ++k) rec0 += static_cast<int>(G.recs[k].size());
             const auto& cm = G.chain_member[gr];
+            const int16_t* const ends[2] = {G.planes[gr].z[0], G.planes[gr].z[kZSixteenths]};  // planes at both ends
             // the k-th line of each orientation under T of every member
             for (int k = 0;; ++k) {
               ZItemDev it{};
               it.rec0 = rec0;
               it.nrec = static_cast<int>(G.recs[gr].size());
               it.flags = T;
+              it.path = path0[vi * ntangs + ti] + static_cast<int>(gr);
               int out = 0, nl = 0, ov = -2;
               for (int s = 0; s < 2 * kZChains; ++s) {
                 it.slot[s] = make_int2(-1, -1);
                 it.owner[s] = static_cast<int8_t>(s);
               }
               for (size_t m = 0; m < cm.size(); ++m) {
-                it.z0[m] = static_cast<int16_t>(G.chain_z0[gr][m]);
-                it.z1[m] = static_cast<int16_t>(G.chain_z1[gr][m]);
                 const int b = (vi * nsegs + cm[m]) * ntangs + ti;
                 const ProjBinDev& pb = h.h_bins[b];
                 int seen[2] = {0, 0};
@@ -152,7 +155,6 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
                 }
               }
               if (nl == 0) break;
-              for (int m = static_cast<int>(cm.size()); m < 8; ++m) it.z0[m] = it.z1[m] = 512;
               // the back projection's buffer: every line's data with the zeros around them that its planes reach, the zeros
               // between two lines shared; first the zeros of the slots without a line
               const int nplanes = planes;
@@ -160,7 +162,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
               for (int s = 0; s < 2 * kZChains; ++s) {
                 if (it.slot[s].x >= 0) continue;
                 const size_t m = static_cast<size_t>(s / 2);
-                const int z0 = m < cm.size() ? G.chain_z0[gr][m] : 512, up = m < cm.size() ? G.chain_z1[gr][m] - z0 : 0;
+                const int z0 = ends[0][m], up = ends[1][m] - z0;
                 // zt = z0 (slot 2 m) or -z0 at the first column (setup_slots), one up or down an event: read from `up`
                 // down to 0, or from 0 up
                 it.boff[s] = static_cast<int16_t>(s % 2 ? -z0 : z0 + up);
@@ -175,7 +177,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
                   int lo = 0, hi = 0;  // planes read below datum 0 and above the last one, by any chain of the line
                   for (size_t m2 = m; m2 < cm.size(); ++m2) {
                     if (cm[m2] != cm[m]) continue;
-                    for (int zr : {G.chain_z0[gr][m2], G.chain_z1[gr][m2]}) {
+                    for (int zr : {ends[0][m2], ends[1][m2]}) {
                       const int zt = (L.flags & 8) ? L.q + 512 - p.min_z - zr : zr - 512 - p.min_z;
                       lo = std::max(lo, zt);
                       hi = std::max(hi, nplanes - 1 - zt - reach);
@@ -225,6 +227,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   }
   h.z_recs.upload(all, h.stream);
   h.z_items.upload(items, h.stream);
+  h.z_planes.upload(sixteenths, h.stream);
   h.dev_status.alloc(1);
   ck(cudaMemsetAsync(h.dev_status.p, 0, sizeof(unsigned), h.stream), "memset");
   ck(cudaStreamSynchronize(h.stream), "path tables");
@@ -233,6 +236,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   z.mean_rec = static_cast<int>(nrecs / std::max<int64_t>(1, ngrp));
   z.recs = h.z_recs.p;
   z.items = h.z_items.p;
+  z.sixteenths = h.z_planes.p;
   h.zparams = z;
   h.z_work.alloc(items.size());
   h.z_partials.alloc(items.size());
@@ -254,6 +258,30 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   h.use_paths = h.use_z = true;
   return true;
 }
+
+// A call with few items leaves most of the GPU's warps idle while each walks hundreds of columns, so the CTA's four warps take
+// a quarter of the path each.  A part repeats the item's set-up, so calls that fill the forward kernel's 16 warps per SM, and
+// short paths, keep a warp an item.  Measured, warp an item / shared: 23 rings, 204 x 204 x 45, one of 21 subsets (OSEM step)
+// 246 / 187 us; 12 rings, 290 x 290 x 23, one of 14 subsets (forward and back) 141 / 55 us; clinical, one of 21 subsets
+// (4140 items, OSEM step) 752 / 860 us.
+constexpr int kZSplitItems = 2368, kZSplitRecords = 64;
+
+// Segments and folds are there for the rounding: a line's sum takes the products of 16 (fold) columns at a time and starts again
+// at every segment, so that no sum is long.  Error of the forward projection against 64 bits (2-norm, one subset), with one sum
+// a path in products of 32 columns / as here: 172 x 172 x 127, 64 rings, span 11 2.5e-7 / 5.9e-8; 344 x 344 x 127 2.4e-7 /
+// 1.1e-7; 171 x 171 x 63 9.7e-8 / 6.1e-8; 101 x 92 x 23 7.2e-8 / 4.9e-8; short paths (34 x 34 x 41) 7.2e-8 / 4.8e-8 with 8 columns
+// (16: 5.2e-8).  The column-staged kernels, which add the sums of 58 columns by eight warps: 1.0e-7, 2.1e-7, 6.9e-8, 5.7e-8,
+// 5.3e-8.  Steep paths of medium length need four segments (two: 1.2e-7 in the first case).  A segment costs 1 to 2 % of the time
+// (all clinical lines: 4.41 ms with one segment in products of 32, 4.71 with four in products of 16).
+ZSplit z_split(const b200rt_projector& h, int n) {
+  const ZParams& z = h.zparams;
+  ZSplit sp;
+  sp.parts = n <= kZSplitItems && z.mean_rec >= kZSplitRecords ? kZWarps : 1;
+  sp.segs = std::max(sp.parts, z.planes == 4 && z.mean_rec >= 64 && z.mean_rec < 256 ? 4 : 2);
+  sp.fold = z.planes > 1 && z.mean_rec < 64 ? 1 : 2;
+  return sp;
+}
+int z_back_parts(const b200rt_projector& h, int n) { return z_split(h, n).parts; }
 
 namespace {
 
@@ -286,9 +314,9 @@ void forward_paths(b200rt_projector& h, const int* list, int n, const float* ima
     return;
   }
   const ZParams& z = h.zparams;
-  const int parts = z_parts(z, n_call >= 0 ? n_call : n);
-  if (z.planes == 1 || !may_alloc) {
-    ck(launch_forward_z(h.params, z, list, n, parts, images, img_stride, 0, out, out_stride, batch, st, ep), "forward projection");
+  const ZSplit sp = z_split(h, n_call >= 0 ? n_call : n);
+  if (z.planes == 1 || !may_alloc || sp.parts > 1) {  // (shared items: few, so a pass over the image costs more than it gives)
+    ck(launch_forward_z(h.params, z, list, n, sp, images, img_stride, 0, out, out_stride, batch, st, ep), "forward projection");
     return;
   }
   const int64_t ncols = static_cast<int64_t>(h.params.ny) * h.params.nx, per = ncols * z_stride(z);
@@ -309,9 +337,9 @@ void forward_paths(b200rt_projector& h, const int* list, int n, const float* ima
     float* o = out ? out + b * out_stride : nullptr;
     if (pad.p) {
       ck(launch_pad_image(x, img_stride, pad.p, per, ncols, h.params.nz, z_stride(z), nb, st), "image planes");
-      ck(launch_forward_z(h.params, z, list, n, parts, pad.p, per, 1, o, out_stride, nb, st, &e), "forward projection");
+      ck(launch_forward_z(h.params, z, list, n, sp, pad.p, per, 1, o, out_stride, nb, st, &e), "forward projection");
     } else {
-      ck(launch_forward_z(h.params, z, list, n, parts, x, img_stride, 0, o, out_stride, nb, st, &e), "forward projection");
+      ck(launch_forward_z(h.params, z, list, n, sp, x, img_stride, 0, o, out_stride, nb, st, &e), "forward projection");
     }
   }
 }
@@ -322,7 +350,7 @@ void back_paths(b200rt_projector& h, const int* list, int n, const float* pd, in
   const int64_t ni = h.geo->image_size();
   if (h.use_z && h.zparams.planes > 1 && n > 0) {
     const ZParams& z = h.zparams;
-    const int parts = z_parts(z, n);
+    const int parts = z_back_parts(h, n);
     const int64_t ncols = static_cast<int64_t>(h.params.ny) * h.params.nx, per = ncols * z_stride(z);
     const int step =
         static_cast<int>(std::min<int64_t>(batch, std::max<int64_t>(1, static_cast<int64_t>(kPadLimit) / per)));
@@ -349,7 +377,7 @@ void add_back_paths(b200rt_projector& h, const int* list, int n, const float* pd
                     int64_t img_stride, int batch, cudaStream_t st, int zero_ends) {
   if (n <= 0) return;
   if (h.use_z)
-    ck(launch_back_z(h.params, h.zparams, list, n, z_parts(h.zparams, n), pd, pd_stride, images, img_stride, 0, batch, st, zero_ends),
+    ck(launch_back_z(h.params, h.zparams, list, n, z_back_parts(h, n), pd, pd_stride, images, img_stride, 0, batch, st, zero_ends),
        "back projection");
   else
     ck(launch_back_paths_atomic_batch(h.params, h.pparams, list, n, pd, pd_stride, images, img_stride, batch, st, zero_ends),
@@ -359,7 +387,7 @@ void add_back_paths(b200rt_projector& h, const int* list, int n, const float* pd
 void back_paths_fixed(b200rt_projector& h, const int* list, int n, const float* pd, unsigned long long* acc,
                       const double* scale, cudaStream_t st, int zero_ends) {
   if (h.use_z)
-    ck(launch_back_z_fixed(h.params, h.zparams, list, n, z_parts(h.zparams, n), pd, acc, scale, st, zero_ends), "back projection");
+    ck(launch_back_z_fixed(h.params, h.zparams, list, n, z_back_parts(h, n), pd, acc, scale, st, zero_ends), "back projection");
   else
     ck(launch_back_paths_fixed(h.params, h.pparams, list, n, pd, acc, scale, st, zero_ends), "back projection");
 }

@@ -182,10 +182,17 @@ void build_path(const std::vector<ZMember>& members, const ZPathLines& fit, int 
         if ((r.op >> m & 1u) && r.w2[m] == 0.f) r.op |= 1u << (6 + m);
       }
     }
+    // the chains' planes where the kernels cut the batches
+    ZPlanes planes;
+    const int nrec = static_cast<int>(recs.size()), nb = (nrec + kZBatch - 1) / kZBatch;
+    for (int m = 0; m < 8; ++m)
+      for (int q = 0, r = 0, zr = m < nc ? cz0[m] : 512; q <= kZSixteenths; ++q) {
+        for (; r < std::min(nb * q / kZSixteenths * kZBatch, nrec); ++r) zr += m < nc ? recs[r].op >> m & 1u : 0;
+        planes.z[q][m] = static_cast<int16_t>(zr);
+      }
+    path.planes.push_back(planes);
     path.recs.push_back(std::move(recs));
     path.chain_member.push_back(std::move(cm));
-    path.chain_z0.push_back(std::move(cz0));
-    path.chain_z1.push_back(std::move(cur));
   }
 }
 

@@ -26,7 +26,7 @@ struct ZPath {
   int total = 0, most = 0;                           // chains of the path, most of one member
   std::vector<std::vector<ZRec>> recs;               // per chain group
   std::vector<std::vector<int>> chain_member;        // per chain group: the member of every chain
-  std::vector<std::vector<int>> chain_z0, chain_z1;  // planes (z + 512) at the first column and at the end
+  std::vector<ZPlanes> planes;                       // per chain group
   bool ok = true;
 };
 

@@ -164,13 +164,20 @@ __device__ __forceinline__ void setup_slots(const ProjParams& p, const ZItemDev&
 }
 
 constexpr int kZRing = 4 * kZBatch;  // records in shared memory
-constexpr int kZAhead = 2;           // columns loaded ahead (forward): at most kZBatch
-constexpr int kZFold = 4;            // batches between two folds (forward)
+// columns loaded ahead (forward), at most 4: more where few warps of an item are to hide the loads, and registers are left
+constexpr int columns_ahead(int NM, int P, bool shared) { return shared && NM * P <= 8 ? 4 : 2; }
 
-// shared memory of a warp: the records' ring, their column offsets, the slots, the lines' values
-__host__ __device__ inline int z_warp_smem(const ZParams& z, bool forward) {
-  return (forward ? kZRing : 2 * kZBatch) * static_cast<int>(sizeof(ZRec) + sizeof(int)) +
-         2 * kZChains * static_cast<int>(sizeof(ZSlot)) + path_align16((forward ? z.max_out : z.max_back) * 4);
+// value buffers of a forward warp: one, or one a segment where the segments' sums are added by several warps
+__host__ __device__ inline int z_buffers(ZSplit sp) { return sp.parts > 1 ? sp.segs / sp.parts : 1; }
+
+// shared memory of a warp: the records' ring, their column offsets, the slots, the lines' values (`buffers` of them) or data
+__host__ __device__ inline int z_forward_smem(const ZParams& z, int buffers) {
+  return kZRing * static_cast<int>(sizeof(ZRec) + sizeof(int)) + 2 * kZChains * static_cast<int>(sizeof(ZSlot)) +
+         path_align16(z.max_out * buffers * 4);
+}
+__host__ __device__ inline int z_back_smem(const ZParams& z) {
+  return 2 * kZBatch * static_cast<int>(sizeof(ZRec) + sizeof(int)) + 2 * kZChains * static_cast<int>(sizeof(ZSlot)) +
+         path_align16(z.max_back * 4);
 }
 
 // The item's records through a ring of batches.  Forward, four: one in use, the next complete with its column offsets
@@ -229,21 +236,6 @@ __device__ __forceinline__ void load_column(const float* __restrict__ img, int o
     for (int j = 0; j < P; ++j) f[j] = z + j < nz ? __ldg(img + off + j) : 0.f;
     c.set(f);
   }
-}
-
-// The events of the records [0, r1), 10 bits a chain: where a warp that takes part of a path starts.
-__device__ __forceinline__ u64 events_before(const ZRec* __restrict__ recs, int r1, int lane) {
-  u64 c = 0;
-  for (int r = lane; r < r1; r += 32) {
-    const uint32_t op = __ldg(&recs[r].op);
-#pragma unroll
-    for (int m = 0; m < kZChains; ++m) c += static_cast<u64>((op >> m) & 1u) << (10 * m);
-  }
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
-  return c;
-}
-__device__ __forceinline__ int chain_plane(const ZItemDev& it, int m, u64 events) {
-  return it.z0[m] + static_cast<int>((events >> (10 * m)) & 1023u);
 }
 
 // what a lane needs at the events: lane 0 has to do with the up line's last plane (what rotates to it leaves there), lane
@@ -418,64 +410,102 @@ struct ZForward {
       G[m].zero();
     }
   }
-  // the sums still in registers (folded), at the chain's last plane
+  // the sums in registers (folded) to the lines' values, the chains at planes zr
   template <int M>
-  __device__ __forceinline__ void flush(const ZSlot* sl, const ZItemDev& it, bool part, u64 events, float* buf, int lane) {
+  __device__ __forceinline__ void flush(const ZSlot* sl, const int16_t* planes, float* buf, int lane) {
     if constexpr (M < NM) {
-      const int zr = part ? chain_plane(it, M, events) : it.z1[M];
+      const int zr = planes[M];
 #pragma unroll
       for (int d = 0; d < 2; ++d) {
         const ZSlot& s = sl[2 * M + d];
-        const int zt = s.zsign * zr + s.zadd;
+        const int z0 = P * lane - (s.zsign * zr + s.zadd), nax = s.nax;
         __syncwarp();
+        if (s.npa == npa_code(1)) {
+          float* v = buf + (s.off + z0);
 #pragma unroll
-        for (int j = 0; j < P; ++j) {
-          const int a = axial_at(P * lane + j - zt, s.npa, s.nax);
-          if (a >= 0) buf[s.off + a] += d ? D[M][j] : U[M][j];
+          for (int j = 0; j < P; ++j)
+            if (static_cast<unsigned>(z0 + j) < static_cast<unsigned>(nax)) v[j] += d ? D[M][j] : U[M][j];
+        } else {
+#pragma unroll
+          for (int j = 0; j < P; ++j) {
+            const int a = axial_at(z0 + j, s.npa, nax);
+            if (a >= 0) buf[s.off + a] += d ? D[M][j] : U[M][j];
+          }
         }
       }
-      flush<M + 1>(sl, it, part, events, buf, lane);
+      flush<M + 1>(sl, planes, buf, lane);
     }
   }
 };
 
-// the lines' values, the sums of `parts` buffers `stride` floats apart in order, through the epilogue by nt threads
-__device__ __forceinline__ void store_values(const ProjParams& p, const ZSlot* sl, int nslots, const float* buf, int stride,
-                                             int parts, int t, int nt, float* __restrict__ out, const FwdEpilogue& ep,
-                                             double& ll, unsigned& ncancel) {
+// the value of one axial position, through the epilogue
+__device__ __forceinline__ void store_value(const ProjParams& p, const ZSlot& s, int a, float v, float* __restrict__ out,
+                                            const FwdEpilogue& ep, double& ll, unsigned& ncancel) {
+  const int seg = s.seg, view = s.view, nax = s.nax;
+  const int64_t i = s.out_base + a;
+  switch (ep.mode) {
+    case kEpiNone: forward_store<kEpiNone>(p, seg, view, 0, nax, i, a, v, out, ep, ll, ncancel); break;
+    case kEpiRatio: forward_store<kEpiRatio>(p, seg, view, 0, nax, i, a, v, out, ep, ll, ncancel); break;
+    case kEpiLoglik: forward_store<kEpiLoglik>(p, seg, view, 0, nax, i, a, v, out, ep, ll, ncancel); break;
+    case kEpiGradient: forward_store<kEpiGradient>(p, seg, view, 0, nax, i, a, v, out, ep, ll, ncancel); break;
+    default: forward_store<kEpiLoglikRatio>(p, seg, view, 0, nax, i, a, v, out, ep, ll, ncancel); break;
+  }
+}
+
+// the lines' values of a warp's item
+__device__ __forceinline__ void store_values(const ProjParams& p, const ZSlot* sl, int nslots, const float* buf, int lane,
+                                             float* __restrict__ out, const FwdEpilogue& ep, double& ll, unsigned& ncancel) {
   for (int k = 0; k < nslots; ++k) {
-    const int nax = sl[k].nax, off = sl[k].off, seg = sl[k].seg, view = sl[k].view;
     if (sl[k].owner != k) continue;
-    const int64_t base = sl[k].out_base;
-    for (int a = t; a < nax; a += nt) {
-      float v = buf[off + a];
-      for (int q = 1; q < parts; ++q) v += buf[q * stride + off + a];
-      switch (ep.mode) {
-        case kEpiNone: forward_store<kEpiNone>(p, seg, view, 0, nax, base + a, a, v, out, ep, ll, ncancel); break;
-        case kEpiRatio: forward_store<kEpiRatio>(p, seg, view, 0, nax, base + a, a, v, out, ep, ll, ncancel); break;
-        case kEpiLoglik: forward_store<kEpiLoglik>(p, seg, view, 0, nax, base + a, a, v, out, ep, ll, ncancel); break;
-        case kEpiGradient: forward_store<kEpiGradient>(p, seg, view, 0, nax, base + a, a, v, out, ep, ll, ncancel); break;
-        default: forward_store<kEpiLoglikRatio>(p, seg, view, 0, nax, base + a, a, v, out, ep, ll, ncancel); break;
-      }
+    for (int a = lane; a < sl[k].nax; a += 32) store_value(p, sl[k], a, buf[sl[k].off + a], out, ep, ll, ncancel);
+  }
+}
+// the same of a shared item: its warps take the lines in turn and add the segments' buffers in order (per of a part, max_out
+// floats each, parts `stride` floats apart; the slots' offsets are those of the last one)
+__device__ __forceinline__ void store_shared(const ProjParams& p, const ZSlot* sl, int nslots, const float* buf, ZSplit sp,
+                                             int part, int per, int max_out, int stride, int lane, float* __restrict__ out,
+                                             const FwdEpilogue& ep, double& ll, unsigned& ncancel) {
+  buf -= part * stride + (per - 1) * max_out;
+  for (int k = part; k < nslots; k += sp.parts) {
+    if (sl[k].owner != k) continue;
+    for (int a = lane; a < sl[k].nax; a += 32) {
+      const float* q = buf + (sl[k].off + a);
+      float v = 0.f;
+      for (int w = 0; w < sp.parts; ++w, q += stride)
+        for (int j = 0; j < per; ++j) v += q[j * max_out];
+      store_value(p, sl[k], a, v, out, ep, ll, ncancel);
     }
   }
 }
 
-// One item by one warp (parts 1), or its path by the CTA's warps in kZWarps parts of the records, whose sums are added
-// before the epilogue: every warp of the CTA calls it then.  smem: the CTA's, warp_smem bytes a warp.
-template <int NM, int P, bool PAD>
-__device__ __forceinline__ void forward_z_item(const ProjParams& p, const ZParams& z, const ZItemDev& it, int parts,
+// the `parts` warps of a CTA that share an item meet
+__device__ __forceinline__ void parts_sync(int warp, int parts) {
+  // (two barriers by number: with one in a register the kernel would take all 16, and fewer CTAs fit on an SM)
+  if (warp < parts)
+    asm volatile("bar.sync 1, %0;" ::"r"(32 * parts) : "memory");
+  else
+    asm volatile("bar.sync 2, %0;" ::"r"(32 * parts) : "memory");
+}
+
+// An item's path in sp.segs segments of its batches, sp.parts warps with as many segments each (1: this warp alone).  A
+// segment's sums go to the lines' values at its end: short sums, so that their rounding stays small, and the same numbers
+// whoever takes the segment where each has a buffer of its own.  smem: this warp's, warp_smem bytes a warp.
+template <int NM, int P, bool PAD, bool SHARED>
+__device__ __forceinline__ void forward_z_item(const ProjParams& p, const ZParams& z, const ZItemDev& it, ZSplit sp,
                                                unsigned char* smem, int warp_smem, const float* __restrict__ img,
                                                float* __restrict__ out, const FwdEpilogue& ep, double& ll,
                                                unsigned& ncancel, int warp, int lane) {
   ZRing<4> rg;
-  rg.init(p, z, it, reinterpret_cast<ZRec*>(smem + warp * warp_smem), PAD ? 32 * P : p.nz);
+  rg.init(p, z, it, reinterpret_cast<ZRec*>(smem), PAD ? 32 * P : p.nz);
   ZSlot* sl = reinterpret_cast<ZSlot*>(rg.offs + kZRing);
   float* buf = reinterpret_cast<float*>(sl + 2 * kZChains);
-  setup_slots(p, it, 2 * NM, sl, buf, lane);
-  for (int i = lane; i < z.max_out; i += 32) buf[i] = 0.f;
+  const int part = SHARED ? warp % sp.parts : 0, per = SHARED ? sp.segs / sp.parts : sp.segs;
+  for (int i = lane; i < z.max_out * (SHARED ? per : 1); i += 32) buf[i] = 0.f;
   const int nb = (it.nrec + kZBatch - 1) / kZBatch;
-  const int b0 = parts > 1 ? nb * warp / parts : 0, b1 = parts > 1 ? nb * (warp + 1) / parts : nb;
+  const int s0 = part * per, s1 = s0 + per;
+  int b = nb * s0 / sp.segs;
+  rg.fetch(b, lane);
+  setup_slots(p, it, 2 * NM, sl, buf, lane);
   const int zlane = P * lane;
   const float* im = img + zlane;
   ZLane k_;
@@ -486,66 +516,77 @@ __device__ __forceinline__ void forward_z_item(const ProjParams& p, const ZParam
   k_.sign = lane == 0 ? -1 : lane == 31 ? 1 : 0;
   ZForward<NM, P> f;
   f.reset();
-  __syncwarp();
-  rg.fetch(b0, lane);
   cp_wait<0>();
   __syncwarp();
-  rg.offsets(b0, lane);
-  rg.fetch(b0 + 1, lane);
+  rg.offsets(b, lane);
+  rg.fetch(b + 1, lane);
   __syncwarp();
-  Planes<P> c[kZAhead];
+  constexpr int kAhead = columns_ahead(NM, P, SHARED);
+  Planes<P> c[kAhead];
 #pragma unroll
-  for (int k = 0; k < kZAhead; ++k) load_column<P, PAD>(im, rg.offs[(b0 & 3) * kZBatch + k], zlane, p.nz, c[k]);
+  for (int k = 0; k < kAhead; ++k) load_column<P, PAD>(im, rg.offs[(b & 3) * kZBatch + k], zlane, p.nz, c[k]);
 #pragma unroll 1
-  for (int bf = b0; bf < b1; bf += kZFold) {
-    const int be = min(bf + kZFold, b1);
+  for (int s = s0; s < s1; ++s) {
+    const int b1 = nb * (s + 1) / sp.segs;
 #pragma unroll 1
-    for (int b = bf; b < be; ++b) {
-      cp_wait<0>();  // batch b + 1, on its way since the batch before
-      __syncwarp();
-      rg.offsets(b + 1, lane);
-      rg.fetch(b + 2, lane);
-      __syncwarp();
-      const ZRec* cur = rg.batch(b);
-      const int n = min(kZBatch, it.nrec - b * kZBatch);
+    while (b < b1) {
+      const int be = min(b + sp.fold, b1);
 #pragma unroll 1
-      for (int k = 0; k < n; k += kZAhead) {
-        // the columns kZAhead on, across the end of the ring
-        const int* ahead = rg.offs + ((b * kZBatch + k + kZAhead) & (kZRing - 1));
+      for (; b < be; ++b) {
+        cp_wait<0>();  // batch b + 1, on its way since the batch before
+        __syncwarp();
+        rg.offsets(b + 1, lane);
+        rg.fetch(b + 2, lane);
+        __syncwarp();
+        const ZRec* cur = rg.batch(b);
+        const int n = min(kZBatch, it.nrec - b * kZBatch);
+#pragma unroll 1
+        for (int k = 0; k < n; k += kAhead) {
+          // the columns kAhead on, across the end of the ring
+          const int* ahead = rg.offs + ((b * kZBatch + k + kAhead) & (kZRing - 1));
 #pragma unroll
-        for (int i = 0; i < kZAhead; ++i) {
-          f.column(cur + k + i, c[i], k_);
-          load_column<P, PAD>(im, ahead[i], zlane, p.nz, c[i]);
+          for (int i = 0; i < kAhead; ++i) {
+            f.column(cur + k + i, c[i], k_);
+            load_column<P, PAD>(im, ahead[i], zlane, p.nz, c[i]);
+          }
         }
       }
+      f.fold();
     }
-    f.fold();
+    f.template flush<0>(sl, z.sixteenths[it.path].z[kZSixteenths / sp.segs * (s + 1)], buf, lane);
+    f.reset();
+    if (SHARED && s + 1 < s1) {  // on to the next segment's buffer
+      __syncwarp();
+      if (lane < 2 * NM) {
+        sl[lane].off += z.max_out;
+        if (sl[lane].addr) sl[lane].addr += 4 * z.max_out;
+      }
+      __syncwarp();
+    }
   }
   cp_wait<0>();
-  const u64 ev = parts > 1 ? events_before(rg.src, min(b1 * kZBatch, it.nrec), lane) : 0;
-  f.template flush<0>(sl, it, parts > 1, ev, buf, lane);
-  if (parts > 1) {
-    __syncthreads();
-    store_values(p, sl, 2 * NM, buf - warp * (warp_smem / 4), warp_smem / 4, parts, threadIdx.x, kZWarps * 32, out, ep, ll,
-                 ncancel);
+  if constexpr (SHARED) {
+    parts_sync(warp, sp.parts);
+    store_shared(p, sl, 2 * NM, buf, sp, part, per, z.max_out, warp_smem / 4, lane, out, ep, ll, ncancel);
   } else {
     __syncwarp();
-    store_values(p, sl, 2 * NM, buf, 0, 1, lane, 32, out, ep, ll, ncancel);
+    store_values(p, sl, 2 * NM, buf, lane, out, ep, ll, ncancel);
   }
 }
 
 // CTAs per SM the forward kernels are compiled for
 constexpr int forward_ctas(int NM, int P) { return P == 4 ? (NM > 4 ? 4 : 5) : P == 2 ? 6 : 7; }
 
-template <int NM, int P, bool PAD>
-__global__ void __launch_bounds__(kZWarps * 32, forward_ctas(NM, P))
-    forward_z_kernel(ProjParams p, ZParams z, const int* __restrict__ list, int n, int parts, const float* __restrict__ img,
+// W: the CTA's warps, kZWarps or (a few items shared by more warps each) up to kZManyWarps
+template <int NM, int P, bool PAD, bool SHARED, int W>
+__global__ void __launch_bounds__(W * 32, W == kZWarps ? forward_ctas(NM, P) : 1)
+    forward_z_kernel(ProjParams p, ZParams z, const int* __restrict__ list, int n, ZSplit sp, const float* __restrict__ img,
                      int64_t img_stride, float* __restrict__ out, int64_t out_stride, FwdEpilogue ep) {
   extern __shared__ __align__(16) unsigned char smem[];
   // one warp's values are the same in all its lanes, which the compiler takes from the broadcast
   const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int i = parts > 1 ? blockIdx.x : blockIdx.x * kZWarps + warp;
-  if (i >= n) return;  // whole warps, or the whole CTA where its warps share an item
+  const int i = SHARED ? (blockIdx.x * (blockDim.x >> 5) + warp) / sp.parts : blockIdx.x * W + warp;
+  if (i >= n) return;  // all the warps of an item
   if (blockIdx.y > 0) {  // image blockIdx.y of a batch
     const int64_t b = blockIdx.y;
     img += b * img_stride;
@@ -557,7 +598,8 @@ __global__ void __launch_bounds__(kZWarps * 32, forward_ctas(NM, P))
   }
   double ll = 0.0;
   unsigned ncancel = 0;
-  forward_z_item<NM, P, PAD>(p, z, z.items[list[i]], parts, smem, z_warp_smem(z, true), img, out, ep, ll, ncancel, warp,
+  const int warp_smem = z_forward_smem(z, z_buffers(sp));
+  forward_z_item<NM, P, PAD, SHARED>(p, z, z.items[list[i]], sp, smem + warp * warp_smem, warp_smem, img, out, ep, ll, ncancel, warp,
                              lane);
   if (ep.mode == kEpiRatio || ep.mode == kEpiGradient || ep.mode == kEpiLoglikRatio) {
     // cancelled singularities (distributable.cxx:590-594)
@@ -567,13 +609,13 @@ __global__ void __launch_bounds__(kZWarps * 32, forward_ctas(NM, P))
   if (ep.mode == kEpiLoglik || ep.mode == kEpiLoglikRatio) {
     // one partial sum per item, reduced in a fixed order by the caller: deterministic
     for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(kFull, ll, o);
-    if (parts > 1) {
-      __shared__ double red[kZWarps];
+    if constexpr (SHARED) {
+      __shared__ double red[W];
       if (lane == 0) red[warp] = ll;
-      __syncthreads();
+      parts_sync(warp, sp.parts);
+      if (warp % sp.parts) return;
       ll = 0.0;
-      for (int w = 0; w < kZWarps; ++w) ll += red[w];
-      if (warp > 0) return;
+      for (int w = 0; w < sp.parts; ++w) ll += red[warp + w];
     }
     if (lane == 0) ep.partials[static_cast<int64_t>(blockIdx.y) * n + i] = ll;
   }
@@ -613,9 +655,9 @@ struct ZBack {
   uint32_t U[NM], D[NM];  // shared addresses of the lines' datum for plane `lane`
 
   template <int M>
-  __device__ __forceinline__ void init(const ZSlot* sl, const ZItemDev& it, u64 events, uint32_t buf, int lane) {
+  __device__ __forceinline__ void init(const ZSlot* sl, const ZItemDev& it, const int16_t* planes, uint32_t buf, int lane) {
     if constexpr (M < NM) {
-      const int zr = chain_plane(it, M, events);
+      const int zr = planes[M];
       U[M] = buf + 4 * (it.boff[2 * M] + lane - (sl[2 * M].zsign * zr + sl[2 * M].zadd));
       D[M] = buf + 4 * (it.boff[2 * M + 1] + lane - (sl[2 * M + 1].zsign * zr + sl[2 * M + 1].zadd));
       float e[P];
@@ -627,7 +669,7 @@ struct ZBack {
         e[j] = a + b;
       }
       E[M].set(e);
-      init<M + 1>(sl, it, events, buf, lane);
+      init<M + 1>(sl, it, planes, buf, lane);
     }
   }
   // chain M's event where its bit is set (the branch in the assembly: see ZForward): E one plane on, and the column's
@@ -732,10 +774,9 @@ __device__ __forceinline__ void back_z_item(const ProjParams& p, const ZParams& 
       buf[off + a * npa] = d;
     }
   }
-  const u64 ev = part > 0 ? events_before(rg.src, b0 * kZBatch, lane) : 0;
   __syncwarp();
   ZBack<NM, P> f;
-  f.template init<0>(sl, it, ev, smem_addr(buf), lane);
+  f.template init<0>(sl, it, z.sixteenths[it.path].z[kZSixteenths / parts * part], smem_addr(buf), lane);
 #pragma unroll 1
   for (int b = b0; b < b1; ++b) {
     cp_wait<0>();
@@ -771,20 +812,20 @@ __global__ void __launch_bounds__(kZWarps * 32, back_ctas(P))
   extern __shared__ __align__(16) unsigned char smem[];
   // one warp's values are the same in all its lanes, which the compiler takes from the broadcast
   const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int i = parts > 1 ? blockIdx.x : blockIdx.x * kZWarps + warp;
+  const int w = blockIdx.x * kZWarps + warp, i = w / parts;
   if (i >= n) return;
-  ZRec* ring = reinterpret_cast<ZRec*>(smem + warp * z_warp_smem(z, false));
+  ZRec* ring = reinterpret_cast<ZRec*>(smem + warp * z_back_smem(z));
   Sink sink = sink0;
   sink.load();
   if (blockIdx.y > 0) {  // image blockIdx.y of a batch
     if (pd) pd += static_cast<int64_t>(blockIdx.y) * pd_stride;
     sink.batch(static_cast<int64_t>(blockIdx.y) * img_stride);
   }
-  back_z_item<NM, P, Sink>(p, z, z.items[list[i]], ring, parts > 1 ? warp : 0, parts, pd, sink, stride, zero_ends, lane);
+  back_z_item<NM, P, Sink>(p, z, z.items[list[i]], ring, w % parts, parts, pd, sink, stride, zero_ends, lane);
 }
 
 // ---- batched reconstructions: persistent CTAs over units of kZWarps (frame, item) work items of one frame ----------------
-// A unit holds kZWarps items (bin -1: none), or one item kZWarps times (kZShared) where its warps share it.
+// A unit holds kZWarps entries: items (bin -1: none), or items repeated for each of the warps that share one.
 
 // the CTA's next unit, or -1
 __device__ __forceinline__ int next_z_unit(unsigned* counter, int nunits) {
@@ -805,13 +846,19 @@ __global__ void __launch_bounds__(kZWarps * 32, forward_ctas(NM, P))
   for (int k; (k = next_z_unit(counter, nunits)) >= 0;) {
     const BatchItem wi = items[k * kZWarps + warp];
     if (wi.bin < 0) continue;
-    const BatchFrameDev& f = frames[wi.frame & ~kZShared];
+    const BatchFrameDev& f = frames[z_frame_of(wi.frame)];
     const ZParams& z = zgeoms[f.geom];
     double ll = 0.0;
     unsigned ncancel = 0;
     constexpr bool kPad = P > 1;
-    forward_z_item<NM, P, kPad>(geoms[f.geom], z, z.items[wi.bin], (wi.frame & kZShared) ? kZWarps : 1, smem, warp_smem, kPad ? f.xpad : f.x, f.ratio,
-                                f.ep, ll, ncancel, warp, lane);
+    const ZSplit sp = z_split_of(wi.frame);
+    const float* x = kPad ? f.xpad : f.x;
+    if (sp.parts > 1)
+      forward_z_item<NM, P, kPad, true>(geoms[f.geom], z, z.items[wi.bin], sp, smem + warp * warp_smem, warp_smem, x, f.ratio,
+                                        f.ep, ll, ncancel, warp, lane);
+    else
+      forward_z_item<NM, P, kPad, false>(geoms[f.geom], z, z.items[wi.bin], sp, smem + warp * warp_smem, warp_smem, x, f.ratio,
+                                         f.ep, ll, ncancel, warp, lane);
     for (int o = 16; o > 0; o >>= 1) ncancel += __shfl_xor_sync(kFull, ncancel, o);
     if (lane == 0 && ncancel && f.ep.cancelled) atomicAdd(f.ep.cancelled, ncancel);
   }
@@ -828,10 +875,10 @@ __global__ void __launch_bounds__(kZWarps * 32, back_ctas(P))
   for (int k; (k = next_z_unit(counter, nunits)) >= 0;) {
     const BatchItem wi = items[k * kZWarps + warp];
     if (wi.bin < 0) continue;
-    const BatchFrameDev& f = frames[wi.frame & ~kZShared];
+    const BatchFrameDev& f = frames[z_frame_of(wi.frame)];
     const ProjParams& p = geoms[f.geom];
     const ZParams& z = zgeoms[f.geom];
-    const int parts = (wi.frame & kZShared) ? kZWarps : 1, part = parts > 1 ? warp : 0;
+    const int parts = z_split_of(wi.frame).parts, part = warp % parts;
     if (f.acc64) {  // a deterministic frame: the same fixed-point integers as its own back projection
       ZFixedSink sink{f.acc64, f.fixed_scale, 0.f};
       sink.load();
@@ -845,17 +892,20 @@ __global__ void __launch_bounds__(kZWarps * 32, back_ctas(P))
 }
 
 template <typename K, typename... A>
-cudaError_t launch_z(K kernel, int sm, int n, int parts, int batch, cudaStream_t st, A... args) {
-  if (n <= 0 || batch <= 0) return cudaSuccess;
+cudaError_t launch_z(K kernel, int sm, int ctas, int warps, int batch, cudaStream_t st, A... args) {
+  if (ctas <= 0 || batch <= 0) return cudaSuccess;
   if (batch > 65535) return cudaErrorInvalidValue;
   if (sm > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess) return e;
   }
-  kernel<<<dim3(parts > 1 ? n : (n + kZWarps - 1) / kZWarps, batch), kZWarps * 32, sm, st>>>(args...);
+  kernel<<<dim3(ctas, batch), warps * 32, sm, st>>>(args...);
   return cudaGetLastError();
 }
+
+// CTAs of kZWarps warps for n items shared by `parts` warps each
+int z_ctas(int n, int parts) { return static_cast<int>((static_cast<int64_t>(n) * parts + kZWarps - 1) / kZWarps); }
 
 // planes of a column, four per thread: rows of `stride` floats from / to rows of nz
 __global__ void pad_image_kernel(const float* __restrict__ in, int64_t in_stride, float* __restrict__ out,
@@ -931,40 +981,51 @@ cudaError_t launch_unpad_image(const float* in, int64_t in_stride, float* out, i
   return cudaGetLastError();
 }
 
-cudaError_t launch_forward_z(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* image,
+cudaError_t launch_forward_z(const ProjParams& p, const ZParams& z, const int* list, int n, ZSplit sp, const float* image,
                              int64_t img_stride, int padded, float* out, int64_t out_stride, int batch,
                              cudaStream_t st, const FwdEpilogue* ep) {
   FwdEpilogue e{};
   if (ep) e = *ep;
-  const int sm = kZWarps * z_warp_smem(z, true);
+  const int sm = z_forward_smem(z, z_buffers(sp));
+  if (padded && sp.parts > 1) return cudaErrorInvalidValue;
   return z_variant(z, [&]<int NM, int P>() {
+    auto run = [&](auto kernel, int ctas, int warps) {
+      return launch_z(kernel, warps * sm, ctas, warps, batch, st, p, z, list, n, sp, image, img_stride, out, out_stride, e);
+    };
+    if (sp.parts > kZWarps) return run(forward_z_kernel<NM, P, false, true, kZManyWarps>, n, sp.parts);
+    if (sp.parts > 1) return run(forward_z_kernel<NM, P, false, true, kZWarps>, z_ctas(n, sp.parts), kZWarps);
     if constexpr (P > 1) {
-      if (padded)
-        return launch_z(forward_z_kernel<NM, P, true>, sm, n, parts, batch, st, p, z, list, n, parts, image, img_stride, out,
-                        out_stride, e);
+      if (padded) return run(forward_z_kernel<NM, P, true, false, kZWarps>, z_ctas(n, 1), kZWarps);
     }
-    return launch_z(forward_z_kernel<NM, P, false>, sm, n, parts, batch, st, p, z, list, n, parts, image, img_stride, out, out_stride,
-                    e);
+    return run(forward_z_kernel<NM, P, false, false, kZWarps>, z_ctas(n, 1), kZWarps);
   });
 }
 
 cudaError_t launch_back_z(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* pd,
-                          int64_t pd_stride,
-                          float* image, int64_t img_stride, int padded, int batch, cudaStream_t st, int zero_ends) {
+                          int64_t pd_stride, float* image, int64_t img_stride, int padded, int batch, cudaStream_t st,
+                          int zero_ends) {
   return z_variant(z, [&]<int NM, int P>() {
-    const int sm = kZWarps * z_warp_smem(z, false);
+    auto run = [&](auto kernel, auto sink, int stride) {
+      return launch_z(kernel, kZWarps * z_back_smem(z), z_ctas(n, parts), kZWarps, batch, st, p, z, list, n, parts, pd,
+                      pd_stride, sink, img_stride, stride, zero_ends);
+    };
     if constexpr (P > 1) {
-      if (padded)
-        return launch_z(back_z_kernel<NM, P, ZFloatSink<true>>, sm, n, parts, batch, st, p, z, list, n, parts, pd, pd_stride,
-                        ZFloatSink<true>{image}, img_stride, z_stride(z), zero_ends);
+      if (padded) return run(back_z_kernel<NM, P, ZFloatSink<true>>, ZFloatSink<true>{image}, z_stride(z));
     }
-    return launch_z(back_z_kernel<NM, P, ZFloatSink<false>>, sm, n, parts, batch, st, p, z, list, n, parts, pd, pd_stride,
-                    ZFloatSink<false>{image}, img_stride, p.nz, zero_ends);
+    return run(back_z_kernel<NM, P, ZFloatSink<false>>, ZFloatSink<false>{image}, p.nz);
+  });
+}
+
+cudaError_t launch_back_z_fixed(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* pd,
+                                unsigned long long* acc, const double* scale, cudaStream_t st, int zero_ends) {
+  return z_variant(z, [&]<int NM, int P>() {
+    return launch_z(back_z_kernel<NM, P, ZFixedSink>, kZWarps * z_back_smem(z), z_ctas(n, parts), kZWarps, 1, st, p, z, list, n,
+                    parts, pd, int64_t(0), ZFixedSink{acc, scale, 0.f}, int64_t(0), p.nz, zero_ends);
   });
 }
 
 int z_batch_smem(const ZParams& z, bool forward) {
-  return kZWarps * z_warp_smem(z, forward);
+  return kZWarps * (forward ? z_forward_smem(z, kZBatchBuffers) : z_back_smem(z));
 }
 
 cudaError_t launch_z_batch(const ZParams& z, bool forward, const ProjParams* geoms, const ZParams* zgeoms,
@@ -997,14 +1058,6 @@ int z_batch_max_ctas_per_sm(const ZParams& z, bool forward, int smem) {
   const cudaError_t e = forward ? z_variant(z, [&]<int NM, int P>() { return count(forward_z_batch_kernel<NM, P>); })
                                 : z_variant(z, [&]<int NM, int P>() { return count(back_z_batch_kernel<NM, P>); });
   return e == cudaSuccess ? n : 0;
-}
-
-cudaError_t launch_back_z_fixed(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* pd,
-                                unsigned long long* acc, const double* scale, cudaStream_t st, int zero_ends) {
-  return z_variant(z, [&]<int NM, int P>() {
-    return launch_z(back_z_kernel<NM, P, ZFixedSink>, kZWarps * z_warp_smem(z, false), n, parts, 1, st, p, z, list, n, parts, pd,
-                    int64_t(0), ZFixedSink{acc, scale, 0.f}, int64_t(0), p.nz, zero_ends);
-  });
 }
 
 }  // namespace b200

@@ -33,15 +33,22 @@ constexpr uint32_t kZGuard = 1u << 12;
 struct ZItemDev {
   int rec0, nrec;       // the path group's records (nrec a multiple of 4)
   int flags;            // T: bit 0 swap x/y, bit 1 negate x, bit 2 negate y
-  int pad;
-  int16_t z0[8], z1[8];  // stored plane (z + 512) of each chain at the first column and at the end
+  int path;             // the path group's planes (ZParams::sixteenths)
   int2 slot[2 * kZChains];         // (index into lines[], basic bin) or (-1, -1)
   int16_t boff[2 * kZChains];      // back projection: the slot's datum 0 in the item's shared buffer (max_back floats)
   int8_t owner[4 * ((2 * kZChains + 3) / 4)];  // the slot whose sums this one shares (two chains of one line)
 };
 
+// stored plane (z + 512) of each chain of a path group before each sixteenth of its batches, where a warp may take over, and
+// at the end
+constexpr int kZSixteenths = 16;
+struct ZPlanes {
+  int16_t z[kZSixteenths + 1][8];
+};
+
 struct ZParams {
   const ZRec* recs;
+  const ZPlanes* sixteenths;
   const ZItemDev* items;
   int nm;         // chains per item the kernels are compiled for: 4 or 6
   int planes;     // planes per lane: 1, 2 or 4 (32 x planes >= nz)
@@ -50,13 +57,15 @@ struct ZParams {
   int max_back;   // longest shared buffer of an item's data with the zeros around them
 };
 
-// Warps that share an item of a call with n items: a call with few items leaves most of the GPU's warps idle while each
-// walks hundreds of columns, so the CTA's four warps take a quarter of the path each.  A part repeats the item's set-up, so
-// calls that fill the forward kernel's 16 warps per SM, and short paths, keep a warp an item.  Measured, warp an item /
-// shared: 23 rings, 204 x 204 x 45, one of 21 subsets (OSEM step) 246 / 187 us; 12 rings, 290 x 290 x 23, one of 14
-// subsets (forward and back) 141 / 55 us; clinical, one of 21 subsets (4140 items, OSEM step) 752 / 860 us.
-constexpr int kZSplitItems = 2368, kZSplitRecords = 64;
-inline int z_parts(const ZParams& z, int n) { return n <= kZSplitItems && z.mean_rec >= kZSplitRecords ? kZWarps : 1; }
+// How a call's items are walked: the forward projection sums an item's path in `segs` segments, taken by `parts` warps, and
+// the back projection's warps take a part each.  The results depend on segs (and on parts = 1 or more), not on how many
+// warps take the segments.
+struct ZSplit {
+  int segs, parts;
+  int fold;  // batches whose products are summed by themselves
+};
+constexpr int kZManyWarps = kZSixteenths;  // most warps of an item
+constexpr int kZBatchBuffers = kZManyWarps / kZWarps;  // value buffers of a warp in the batched kernels, whose CTAs have kZWarps warps
 
 // column stride (floats) of the padded images the kernels use when planes > 1
 inline int z_stride(const ZParams& z) { return 32 * z.planes; }
@@ -67,8 +76,9 @@ cudaError_t launch_pad_image(const float* in, int64_t in_stride, float* out, int
 cudaError_t launch_unpad_image(const float* in, int64_t in_stride, float* out, int64_t out_stride, int64_t ncols, int nz,
                                int stride, int batch, cudaStream_t st);
 
-// padded != 0: image has column stride z_stride(z) (16-byte aligned), else nz
-cudaError_t launch_forward_z(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* image,
+// padded != 0: image has column stride z_stride(z) (16-byte aligned), else nz; the forward projection takes padded images
+// with sp.parts = 1 only
+cudaError_t launch_forward_z(const ProjParams& p, const ZParams& z, const int* list, int n, ZSplit sp, const float* image,
                              int64_t img_stride, int padded, float* out, int64_t out_stride, int batch, cudaStream_t st,
                              const FwdEpilogue* ep);
 cudaError_t launch_back_z(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* pd, int64_t pd_stride,
@@ -81,7 +91,20 @@ cudaError_t launch_back_z_fixed(const ProjParams& p, const ZParams& z, const int
 inline bool z_same_variant(const ZParams& a, const ZParams& b) {
   return a.nm == b.nm && a.planes == b.planes;
 }
-constexpr int kZShared = 1 << 30;  // BatchItem::frame: the unit's entries are one item, shared by its warps
+// BatchItem::frame with the split of the frame's items: the frame in the low 20 bits, log2 of segs, parts, fold above it
+constexpr int kZFrameBits = 20;
+__host__ __device__ inline int z_frame_of(int f) { return f & ((1 << kZFrameBits) - 1); }
+__host__ __device__ inline ZSplit z_split_of(int f) {
+  return ZSplit{1 << (f >> 20 & 7), 1 << (f >> 23 & 7), 1 << (f >> 26 & 7)};
+}
+inline int z_frame_split(int frame, ZSplit sp) {
+  auto lg = [](int v) {
+    int k = 0;
+    while (1 << k < v) ++k;
+    return k;
+  };
+  return frame | lg(sp.segs) << 20 | lg(sp.parts) << 23 | lg(sp.fold) << 26;
+}
 int z_batch_smem(const ZParams& z, bool forward);
 int z_batch_max_ctas_per_sm(const ZParams& z, bool forward, int smem);
 cudaError_t launch_z_batch(const ZParams& z, bool forward, const ProjParams* geoms, const ZParams* zgeoms,
