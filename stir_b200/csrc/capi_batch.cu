@@ -116,6 +116,18 @@ void use_family(b200rt_batch& b, int kernels) {
 }
 
 // device tables and per-frame scratch; done once after the last add_frame
+// most value buffers that a warp needs for the items of geometry gi's frames
+int value_buffers(const b200rt_batch& b, int gi) {
+  int most = 1;
+  for (const auto& f : b.frames) {
+    if (f->geom != gi) continue;
+    std::vector<int> items(f->nsub, 0);
+    for (int v : f->h->h_item_view) ++items[v % f->nsub];
+    for (int n : items) most = std::max(most, b200::z_buffers(b200::z_batch_split(z_split(*f->h, n))));
+  }
+  return most;
+}
+
 void batch_finalize(b200rt_batch& b) {
   if (b.ready) return;
   std::vector<b200::ProjParams> gp;
@@ -158,8 +170,8 @@ void batch_finalize(b200rt_batch& b) {
       zg.push_back(h->zparams);
       int smem[2];
       if (h->use_z) {
-        smem[0] = b200::z_batch_smem(h->zparams, true);
-        smem[1] = b200::z_batch_smem(h->zparams, false);
+        smem[0] = b200::z_batch_smem(h->zparams, true, value_buffers(b, static_cast<int>(gi)));
+        smem[1] = b200::z_batch_smem(h->zparams, false, 1);
       } else {
         smem[0] = b200::path_smem_fwd(pp.K, h->params.nz, pp.zpad, pp.max_lines, pp.max_acc, pp.npa_max).total;
         smem[1] = b200::path_smem_back(h->params.nz, pp.max_lines, pp.max_members, pp.nax_max, pp.npa_max).total;
@@ -324,8 +336,8 @@ const BatchItem* batch_items(b200rt_batch& b, int k, int order, int& count) {
     int parts = 1, code = frame;
     if (zf) {
       if (frame >> b200::kZFrameBits) throw std::invalid_argument("too many batched frames");
-      b200::ZSplit sp = z_split(h, static_cast<int>(per_frame[fi].size()));
-      parts = sp.parts = std::min(sp.parts, b200::kZWarps);
+      const b200::ZSplit sp = b200::z_batch_split(z_split(h, static_cast<int>(per_frame[fi].size())));
+      parts = sp.parts;
       code = b200::z_frame_split(frame, sp);
     }
     for (int bin : per_frame[fi])

@@ -259,12 +259,38 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   return true;
 }
 
-// A call with few items leaves most of the GPU's warps idle while each walks hundreds of columns, so the CTA's four warps take
-// a quarter of the path each.  A part repeats the item's set-up, so calls that fill the forward kernel's 16 warps per SM, and
-// short paths, keep a warp an item.  Measured, warp an item / shared: 23 rings, 204 x 204 x 45, one of 21 subsets (OSEM step)
-// 246 / 187 us; 12 rings, 290 x 290 x 23, one of 14 subsets (forward and back) 141 / 55 us; clinical, one of 21 subsets
-// (4140 items, OSEM step) 752 / 860 us.
-constexpr int kZSplitItems = 2368, kZSplitRecords = 64;
+namespace {
+
+// Warps that share each of n items with paths of `rec` records, `resident` warps on the GPU at a time.  A call with few items
+// leaves most of the GPU idle while each warp walks its path, so the warps are doubled while what they add runs beside the
+// others (m: warps wanted over resident ones) and a part still has enough records for its set-up (list, item, lines, the first
+// records: about what 20 records cost).  Measured, us, one image: forward 1 / 2 / 4 / 8 / 16 warps an item, 62 items of 152
+// records 42 / 22 / 13.5 / 10.4 / 10.3; 438 of 83 30 / 18 / 12.4 / 10.4 / 16.5; 630 of 146 37 / 21 / 13.5 / 16.5 / 23; 1972 of 173
+// 45 / 27 / 27 / 37; 3423 of 391 97 / 72 / 66 / 80; 4158 of 68 27 / 29 / 33; 15892 of 355 282 / 268 / 288; 49350 of 49 196 / 243.
+// Back: 243 of 241 70 / 41 / 27 / 19 / 16.5; 833 of 175 53 / 33 / 24 / 21 / 25; 2618 of 65 28 / 20 / 22 / 28; 4158 of 68 26 / 27 / 30.
+// `far`: also worth it where each warp's own latency is what bounds it (long paths, few registers)
+int sharing_warps(int n, int rec, int resident, bool far) {
+  int parts = 1;
+  while (parts < kZManyWarps) {
+    const int next = 2 * parts;
+    const double m = static_cast<double>(n) * next / resident;
+    const int r = rec / next;
+    const bool ok = m <= 1.0                ? r >= 5
+                    : next >= 8             ? false
+                    : m <= 1.5              ? r >= 16
+                    : m <= 2.3              ? r >= 30
+                    : far && m <= 4.0       ? r >= 90
+                    : far && m <= 12.0      ? next == 2 && r >= 125
+                                            : false;
+    if (!ok) break;
+    parts = next;
+  }
+  return parts;
+}
+
+constexpr int kSharedLimit = 200 * 1024;
+
+}  // namespace
 
 // Segments and folds are there for the rounding: a line's sum takes the products of 16 (fold) columns at a time and starts again
 // at every segment, so that no sum is long.  Error of the forward projection against 64 bits (2-norm, one subset), with one sum
@@ -276,12 +302,39 @@ constexpr int kZSplitItems = 2368, kZSplitRecords = 64;
 ZSplit z_split(const b200rt_projector& h, int n) {
   const ZParams& z = h.zparams;
   ZSplit sp;
-  sp.parts = n <= kZSplitItems && z.mean_rec >= kZSplitRecords ? kZWarps : 1;
+  sp.parts = sharing_warps(n, z.mean_rec, z_resident_warps(z, true), z.planes == 1 || (z.planes == 2 && z.nm == 4));
+  // 16 warps a CTA: two CTAs an SM where the registers allow it, one elsewhere
+  if (sp.parts == 16 && n > 148 && (z.nm > 4 || z.planes == 4)) sp.parts = 8;
+  while (sp.parts > 1 && std::max(sp.parts, kZWarps) * z_forward_smem(z, 2) > kSharedLimit) sp.parts /= 2;
   sp.segs = std::max(sp.parts, z.planes == 4 && z.mean_rec >= 64 && z.mean_rec < 256 ? 4 : 2);
   sp.fold = z.planes > 1 && z.mean_rec < 64 ? 1 : 2;
   return sp;
 }
-int z_back_parts(const b200rt_projector& h, int n) { return z_split(h, n).parts; }
+int z_back_parts(const b200rt_projector& h, int n) {
+  return sharing_warps(n, h.zparams.mean_rec, z_resident_warps(h.zparams, false), h.zparams.planes == 1);
+}
+
+// Whether a call is worth padded images, which save instructions and cache lines per column walked and cost a pass over the
+// image each way, the launches and an allocation.  Forward, one warp an item, padded / plain, us: clinical, one of 21 subsets (4140
+// items of 373 records, 118336 columns) 291 / 298, all lines 4694 / 5290; 4117 items of 218 records, 62500 columns 166 / 169;
+// 742 of 245, 109392 columns 112 / 119 and shared 56 / 39; two planes a lane: 41356 of 181, 29241 columns 606 / 623; 9312 of
+// 259, 111556 columns 188 / 177; 4032 of 145, 15776 columns 73 / 69.
+bool pad_forward(const b200rt_projector& h, int n, int batch) {
+  const ZParams& z = h.zparams;
+  const int64_t ncols = static_cast<int64_t>(h.params.ny) * h.params.nx * batch;
+  const int64_t walked = static_cast<int64_t>(n) * z.mean_rec * batch;
+  return z.planes == 4 ? walked >= 200000 + 8 * ncols : z.planes == 2 && walked >= 1000000 + 20 * ncols;
+}
+// Back, where the planes fill the lanes (a plain column has a reduction for every 32 planes or part of them, a padded one for
+// all of the lanes' planes: 79 of 128 planes 1020 / 775 us).  127 of 128 planes: all clinical lines 3635 / 4044, one of 21 subsets 273 /
+// 275; 4950 items of 110 records, 15876 columns 76 / 64; 28050 of 31, 1296 columns 120 / 135; 63 of 64 planes: 41356 of 181 415 /
+// 457; 9312 of 259, 111556 columns 153 / 142.
+bool pad_back(const b200rt_projector& h, int n, int batch) {
+  const ZParams& z = h.zparams;
+  const int64_t ncols = static_cast<int64_t>(h.params.ny) * h.params.nx * batch;
+  const int64_t walked = static_cast<int64_t>(n) * z.mean_rec * batch;
+  return z.planes > 1 && 4 * h.params.nz > 3 * z_stride(z) && walked >= 500000 + 20 * ncols;
+}
 
 namespace {
 
@@ -315,7 +368,7 @@ void forward_paths(b200rt_projector& h, const int* list, int n, const float* ima
   }
   const ZParams& z = h.zparams;
   const ZSplit sp = z_split(h, n_call >= 0 ? n_call : n);
-  if (z.planes == 1 || !may_alloc || sp.parts > 1) {  // (shared items: few, so a pass over the image costs more than it gives)
+  if (!may_alloc || sp.parts > 1 || !pad_forward(h, n_call >= 0 ? n_call : n, batch)) {
     ck(launch_forward_z(h.params, z, list, n, sp, images, img_stride, 0, out, out_stride, batch, st, ep), "forward projection");
     return;
   }
@@ -348,7 +401,7 @@ void forward_paths(b200rt_projector& h, const int* list, int n, const float* ima
 void back_paths(b200rt_projector& h, const int* list, int n, const float* pd, int64_t pd_stride, float* images,
                 int64_t img_stride, int batch, cudaStream_t st, int zero_ends) {
   const int64_t ni = h.geo->image_size();
-  if (h.use_z && h.zparams.planes > 1 && n > 0) {
+  if (h.use_z && n > 0 && pad_back(h, n, batch)) {
     const ZParams& z = h.zparams;
     const int parts = z_back_parts(h, n);
     const int64_t ncols = static_cast<int64_t>(h.params.ny) * h.params.nx, per = ncols * z_stride(z);

@@ -167,15 +167,12 @@ constexpr int kZRing = 4 * kZBatch;  // records in shared memory
 // columns loaded ahead (forward), at most 4: more where few warps of an item are to hide the loads, and registers are left
 constexpr int columns_ahead(int NM, int P, bool shared) { return shared && NM * P <= 8 ? 4 : 2; }
 
-// value buffers of a forward warp: one, or one a segment where the segments' sums are added by several warps
-__host__ __device__ inline int z_buffers(ZSplit sp) { return sp.parts > 1 ? sp.segs / sp.parts : 1; }
-
 // shared memory of a warp: the records' ring, their column offsets, the slots, the lines' values (`buffers` of them) or data
-__host__ __device__ inline int z_forward_smem(const ZParams& z, int buffers) {
+__host__ __device__ inline int forward_smem(const ZParams& z, int buffers) {
   return kZRing * static_cast<int>(sizeof(ZRec) + sizeof(int)) + 2 * kZChains * static_cast<int>(sizeof(ZSlot)) +
          path_align16(z.max_out * buffers * 4);
 }
-__host__ __device__ inline int z_back_smem(const ZParams& z) {
+__host__ __device__ inline int back_smem(const ZParams& z) {
   return 2 * kZBatch * static_cast<int>(sizeof(ZRec) + sizeof(int)) + 2 * kZChains * static_cast<int>(sizeof(ZSlot)) +
          path_align16(z.max_back * 4);
 }
@@ -598,7 +595,7 @@ __global__ void __launch_bounds__(W * 32, W == kZWarps ? forward_ctas(NM, P) : 1
   }
   double ll = 0.0;
   unsigned ncancel = 0;
-  const int warp_smem = z_forward_smem(z, z_buffers(sp));
+  const int warp_smem = forward_smem(z, z_buffers(sp));
   forward_z_item<NM, P, PAD, SHARED>(p, z, z.items[list[i]], sp, smem + warp * warp_smem, warp_smem, img, out, ep, ll, ncancel, warp,
                              lane);
   if (ep.mode == kEpiRatio || ep.mode == kEpiGradient || ep.mode == kEpiLoglikRatio) {
@@ -814,7 +811,7 @@ __global__ void __launch_bounds__(kZWarps * 32, back_ctas(P))
   const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int w = blockIdx.x * kZWarps + warp, i = w / parts;
   if (i >= n) return;
-  ZRec* ring = reinterpret_cast<ZRec*>(smem + warp * z_back_smem(z));
+  ZRec* ring = reinterpret_cast<ZRec*>(smem + warp * back_smem(z));
   Sink sink = sink0;
   sink.load();
   if (blockIdx.y > 0) {  // image blockIdx.y of a batch
@@ -986,7 +983,7 @@ cudaError_t launch_forward_z(const ProjParams& p, const ZParams& z, const int* l
                              cudaStream_t st, const FwdEpilogue* ep) {
   FwdEpilogue e{};
   if (ep) e = *ep;
-  const int sm = z_forward_smem(z, z_buffers(sp));
+  const int sm = forward_smem(z, z_buffers(sp));
   if (padded && sp.parts > 1) return cudaErrorInvalidValue;
   return z_variant(z, [&]<int NM, int P>() {
     auto run = [&](auto kernel, int ctas, int warps) {
@@ -1006,7 +1003,7 @@ cudaError_t launch_back_z(const ProjParams& p, const ZParams& z, const int* list
                           int zero_ends) {
   return z_variant(z, [&]<int NM, int P>() {
     auto run = [&](auto kernel, auto sink, int stride) {
-      return launch_z(kernel, kZWarps * z_back_smem(z), z_ctas(n, parts), kZWarps, batch, st, p, z, list, n, parts, pd,
+      return launch_z(kernel, kZWarps * back_smem(z), z_ctas(n, parts), kZWarps, batch, st, p, z, list, n, parts, pd,
                       pd_stride, sink, img_stride, stride, zero_ends);
     };
     if constexpr (P > 1) {
@@ -1019,13 +1016,18 @@ cudaError_t launch_back_z(const ProjParams& p, const ZParams& z, const int* list
 cudaError_t launch_back_z_fixed(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* pd,
                                 unsigned long long* acc, const double* scale, cudaStream_t st, int zero_ends) {
   return z_variant(z, [&]<int NM, int P>() {
-    return launch_z(back_z_kernel<NM, P, ZFixedSink>, kZWarps * z_back_smem(z), z_ctas(n, parts), kZWarps, 1, st, p, z, list, n,
+    return launch_z(back_z_kernel<NM, P, ZFixedSink>, kZWarps * back_smem(z), z_ctas(n, parts), kZWarps, 1, st, p, z, list, n,
                     parts, pd, int64_t(0), ZFixedSink{acc, scale, 0.f}, int64_t(0), p.nz, zero_ends);
   });
 }
 
-int z_batch_smem(const ZParams& z, bool forward) {
-  return kZWarps * (forward ? z_forward_smem(z, kZBatchBuffers) : z_back_smem(z));
+int z_forward_smem(const ZParams& z, int buffers) { return forward_smem(z, buffers); }
+int z_resident_warps(const ZParams& z, bool forward) {
+  return 148 * kZWarps * (forward ? forward_ctas(z.nm, z.planes) : back_ctas(z.planes));
+}
+
+int z_batch_smem(const ZParams& z, bool forward, int buffers) {
+  return kZWarps * (forward ? forward_smem(z, buffers) : back_smem(z));
 }
 
 cudaError_t launch_z_batch(const ZParams& z, bool forward, const ProjParams* geoms, const ZParams* zgeoms,

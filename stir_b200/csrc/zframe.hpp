@@ -65,7 +65,16 @@ struct ZSplit {
   int fold;  // batches whose products are summed by themselves
 };
 constexpr int kZManyWarps = kZSixteenths;  // most warps of an item
-constexpr int kZBatchBuffers = kZManyWarps / kZWarps;  // value buffers of a warp in the batched kernels, whose CTAs have kZWarps warps
+// value buffers of a forward warp: one, or one a segment where the segments' sums are added by several warps
+__host__ __device__ inline int z_buffers(ZSplit sp) { return sp.parts > 1 ? sp.segs / sp.parts : 1; }
+// the split as the batched kernels take it, whose CTAs have kZWarps warps: the same segments, so the same sums
+inline ZSplit z_batch_split(ZSplit sp) {
+  sp.parts = sp.parts < kZWarps ? sp.parts : kZWarps;
+  return sp;
+}
+// shared memory of a forward warp, and the warps of a projection that the GPU runs at a time
+int z_forward_smem(const ZParams& z, int buffers);
+int z_resident_warps(const ZParams& z, bool forward);
 
 // column stride (floats) of the padded images the kernels use when planes > 1
 inline int z_stride(const ZParams& z) { return 32 * z.planes; }
@@ -105,7 +114,7 @@ inline int z_frame_split(int frame, ZSplit sp) {
   };
   return frame | lg(sp.segs) << 20 | lg(sp.parts) << 23 | lg(sp.fold) << 26;
 }
-int z_batch_smem(const ZParams& z, bool forward);
+int z_batch_smem(const ZParams& z, bool forward, int buffers);
 int z_batch_max_ctas_per_sm(const ZParams& z, bool forward, int smem);
 cudaError_t launch_z_batch(const ZParams& z, bool forward, const ProjParams* geoms, const ZParams* zgeoms,
                            const BatchFrameDev* frames, const BatchItem* items, int nunits, unsigned* counter, int smem,

@@ -10,11 +10,11 @@ from stir_b200 import geometry as G
 pytestmark = pytest.mark.gpu
 
 
-def _geometry(rings, span, delta, dets=64, tang=21, nz=None, ny=23, nx=23, rays=1, planes_per_ring=2):
+def _geometry(rings, span, delta, dets=64, tang=21, nz=None, ny=23, nx=23, rays=1, planes_per_ring=2, vxy=4.1):
     sc = G.Scanner(rings, dets, 100.0, 0.0, 4.0, float(np.float32(np.pi * 100.0 / dets)))
     pdi = G.ProjDataInfoCTI(sc, span, delta, dets // 2, tang)
     nz = nz or planes_per_ring * (rings - 1) + 1
-    img = G.ImageGeometry(nz, ny, nx, (4.0 / planes_per_ring, 4.1, 4.1))
+    img = G.ImageGeometry(nz, ny, nx, (4.0 / planes_per_ring, vxy, vxy))
     return pdi, img, rays
 
 
@@ -112,6 +112,55 @@ def test_calls_on_two_streams(cuda_device):
     for k in range(2):
         for o in outs[k]:
             assert torch.equal(o, ref[k])
+
+
+# Calls with so few items that warps share them: one of many subsets, paths of 20 to 250 columns, with 1, 2 and
+# 4 planes a lane, two rays, several chain groups, 16 warps an item; and the number of subsets
+SHARED = {
+    "1 plane a lane": (_geometry(8, 3, 7, dets=96, tang=40, ny=90, nx=90, vxy=2.00), 12),
+    "1 plane, 16 warps": (_geometry(8, 3, 4, dets=96, tang=12, ny=200, nx=200, vxy=0.90), 24),
+    "1 plane, two rays": (_geometry(9, 3, 7, dets=96, tang=40, ny=84, nx=90, vxy=2.00, rays=2), 12),
+    "1 plane, span 1": (_geometry(8, 1, 7, dets=96, tang=40, ny=85, nx=85, vxy=2.12), 12),
+    "2 planes": (_geometry(21, 5, 17, dets=96, tang=40, ny=80, nx=80, vxy=2.25), 12),
+    "2 planes, two rays": (_geometry(23, 7, 17, dets=96, tang=30, ny=90, nx=71, vxy=2.54, rays=2), 12),
+    "4 planes": (_geometry(40, 7, 30, dets=96, tang=30, ny=91, nx=91, vxy=1.98), 12),
+    "4 planes, two rays": (_geometry(45, 11, 40, dets=96, tang=20, ny=72, nx=72, vxy=2.50, rays=2), 12),
+    "4 planes, 8 warps": (_geometry(50, 11, 16, dets=96, tang=8, ny=190, nx=190, vxy=0.95), 24),
+    "shorter than the parts": (_geometry(8, 3, 7, dets=96, tang=40, ny=19, nx=19), 12),
+}
+
+
+@pytest.mark.parametrize("name", list(SHARED))
+def test_items_shared_by_warps(name, cuda_device):
+    import torch
+    from oracle.oracle import Oracle
+    from stir_b200.projectors import RayTracingProjector
+    from stir_b200.subsets import basic_views_in_subset
+    (pdi, img, rays), nsub = SHARED[name]
+    # at most 8 symmetry operations and 3 chain groups a path: fewer items than half the warps that the GPU runs at a time
+    # (148 x 16), so that two warps share an item where a path has ten records
+    paths = len(basic_views_in_subset(pdi.num_views, 3, 1, nsub)) * (pdi.num_tangential_poss // 2 + 1)
+    assert paths * 8 * 3 <= 148 * 16 // 2 and min(img.nx, img.ny) >= 19
+    proj = RayTracingProjector(pdi, img, num_tangential_LORs=rays, device=cuda_device)
+    orc = Oracle(proj.geometry)
+    x = np.random.default_rng(9).uniform(0.5, 1.5, img.shape).astype(np.float32)
+    xd = proj.image_to_device_layout(torch.from_numpy(x).cuda())
+    y = np.random.default_rng(10).uniform(0.5, 1.5, proj.projdata_size).astype(np.float32)
+    yd = proj.projdata_to_device_layout(torch.from_numpy(y).cuda())
+    for subset in (1, 0):
+        got = proj.projdata_from_device_layout(proj.forward_dev(xd, subset_num=subset, num_subsets=nsub)).cpu().numpy()
+        ref = orc.forward(x, subset, nsub)
+        assert np.all(np.abs(got - ref) <= _bound(orc) * np.abs(ref) + 1e-12)
+        ref = orc.back(y, subset, nsub)
+        for mode in (_abi.BACKPROJECT_ATOMIC, _abi.BACKPROJECT_DETERMINISTIC):
+            got = proj.image_from_device_layout(proj.back_dev(yd, subset_num=subset, num_subsets=nsub, mode=mode)).cpu().numpy()
+            assert np.all(np.abs(got - ref) <= _bound(orc) * np.abs(ref) + 1e-6 * ref.max() * (mode != _abi.BACKPROJECT_ATOMIC))
+    # infinite voxels and data stay in their rows
+    x[img.nz // 2, img.ny // 2, img.nx // 2 + 2] = np.inf
+    got = proj.projdata_from_device_layout(proj.forward_dev(proj.image_to_device_layout(torch.from_numpy(x).cuda()),
+                                                            subset_num=1, num_subsets=nsub)).cpu().numpy()
+    ref = orc.forward(x, 1, nsub)
+    assert not np.isnan(got).any() and np.array_equal(np.isinf(got), np.isinf(ref))
 
 
 def test_forward_sums_are_short(cuda_device):
