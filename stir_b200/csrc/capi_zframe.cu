@@ -70,6 +70,20 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   if (most > kZChains) return false;
   const int ng = (total + kZChains - 1) / kZChains;
   z.nm = std::max((total + ng - 1) / ng, most) <= 4 ? 4 : kZChains;
+  // Several groups of six chains with few elements each, four planes a lane: a record costs the same whether one chain or six
+  // have an element, and the column-staged kernels only pay for the elements.  221 x 222 x 117 image, two rays, three groups,
+  // 2.5 elements a record, one of 4 subsets: forward 844 / 650 us, back 554 / 657; 260 x 260 x 109, three groups, 4.6 elements: 94 /
+  // 107 and 75 / 127.
+  int64_t walked = 0, paths = 0, parts = 0, elements = 0;
+  for (const ZPath& G : groups)
+    if (G.total > 0) {
+      const int n = (G.total + z.nm - 1) / z.nm;
+      ++paths;
+      parts += n;
+      walked += static_cast<int64_t>(G.columns) * n;
+      elements += G.elements;
+    }
+  if (z.planes == 4 && z.nm == kZChains && 2 * parts >= 3 * paths && 5 * elements < 13 * walked) return false;
   run(1, z.nm);
   count();
   if (most > kZChains) return false;

@@ -99,6 +99,8 @@ void build_path(const std::vector<ZMember>& members, const ZPathLines& fit, int 
   }
   path.total = total;
   path.most = most;
+  path.columns = ncols;
+  for (const ZMember& pb : members) path.elements += pb.row_len;
   if (cap == 0 || most > cap) return;  // a record has room for cap chains
   // members into groups of at most cap chains, in order
   std::vector<std::vector<int>> parts;

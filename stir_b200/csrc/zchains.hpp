@@ -24,6 +24,7 @@ struct ZPathLines {
 
 struct ZPath {
   int total = 0, most = 0;                           // chains of the path, most of one member
+  int columns = 0, elements = 0;                     // of all members
   std::vector<std::vector<ZRec>> recs;               // per chain group
   std::vector<std::vector<int>> chain_member;        // per chain group: the member of every chain
   std::vector<ZPlanes> planes;                       // per chain group

@@ -33,6 +33,7 @@ CASES = {
     "span 1, 4 planes a ring": _geometry(9, 1, 5, planes_per_ring=4),
     "truncated segment": _geometry(20, 5, 8),
     "rectangular": _geometry(11, 3, 7, ny=19, nx=31),
+    "sparse chains": _geometry(59, 7, 41, dets=32, tang=11, ny=61, nx=60, vxy=1.1, rays=2),
     "even image": _geometry(10, 7, 9, ny=24, nx=24, tang=24),
 }
 
