@@ -213,6 +213,24 @@ void forward_paths(b200rt_projector& h, const int* list, int n, const float* ima
                    int64_t out_stride, int batch, cudaStream_t st, const FwdEpilogue* ep, bool may_alloc = true, int n_call = -1);
 void back_paths(b200rt_projector& h, const int* list, int n, const float* pd, int64_t pd_stride, float* images,
                 int64_t img_stride, int batch, cudaStream_t st, int zero_ends);
+class BackSums {
+ public:
+  BackSums(b200rt_projector& h, int n, int images, cudaStream_t st);  // n: items of the whole call
+  BackSums(const BackSums&) = delete;
+  ~BackSums();
+  bool own() const { return sums_ != nullptr; }
+  int step() const { return step_; }  // images at a time
+  void clear(int images);
+  void add(const int* list, int n, const float* pd, int64_t pd_stride, int images, int zero_ends);
+  void collect(float* images, int64_t img_stride, int n);
+
+ private:
+  b200rt_projector& h_;
+  cudaStream_t st_;
+  float* sums_ = nullptr;
+  int64_t per_ = 0;  // floats of an image's sums
+  int stride_ = 0, step_ = 1;
+};
 void add_back_paths(b200rt_projector& h, const int* list, int n, const float* pd, int64_t pd_stride, float* images,
                     int64_t img_stride, int batch, cudaStream_t st, int zero_ends);
 void back_paths_fixed(b200rt_projector& h, const int* list, int n, const float* pd, unsigned long long* acc,

@@ -26,9 +26,9 @@ struct b200rt_batch {
     b200rt_prior prior{};
     float prior_w[27] = {0};
     float min_rel = 0.f, max_rel = 0.f;
-    // z-frame geometries: the estimate in padded columns, made before the forward projection, and the numerator (not of
-    // deterministic frames), copied to u after the back projection
-    DevBuf<float> xpad, upad;
+    // z-frame geometries: the estimate in padded columns, made before the forward projection, and the numerator's sums (not
+    // of deterministic frames; BatchFrameDev::usums), collected in u after the back projection
+    DevBuf<float> xpad, usums;
     DevBuf<float> ratio, u, grad, small_value, partial_max, umax;
     DevBuf<unsigned int> cancelled;
     // B200RT_BACKPROJECT_DETERMINISTIC: fixed-point numerator, its scale (from the ratio's bound 1e4 and the
@@ -219,14 +219,17 @@ void batch_finalize(b200rt_batch& b) {
     }
     const size_t padded = static_cast<size_t>(b200::z_stride(f.h->zparams)) * g.desc().ny * g.desc().nx;
     f.xpad.release();
-    f.upad.release();
-    if (paths && f.h->use_z && f.h->zparams.planes > 1) {
-      f.xpad.alloc(padded);
-      if (f.mode != B200RT_BACKPROJECT_DETERMINISTIC) f.upad.alloc(padded);
+    f.usums.release();
+    if (paths && f.h->use_z) {
+      const b200::ZParams& z = f.h->zparams;
+      if (z.planes > 1) f.xpad.alloc(padded);
+      if (f.mode != B200RT_BACKPROJECT_DETERMINISTIC && (z.planes > 1 || z.copies > 1))
+        f.usums.alloc(static_cast<size_t>(b200::z_image_floats(static_cast<int64_t>(g.desc().ny) * g.desc().nx,
+                                                               z.planes > 1 ? b200::z_stride(z) : g.desc().nz)) * z.copies);
     }
     BatchFrameDev d{};
     d.xpad = f.xpad.p;
-    d.upad = f.upad.p;
+    d.usums = f.usums.p;
     d.geom = f.geom;
     d.x = f.x;
     d.ratio = f.ratio.p;
@@ -417,8 +420,8 @@ void batch_zero(b200rt_batch& b, int k, cudaStream_t st) {
     ck(cudaMemsetAsync(f.cancelled.p, 0, sizeof(unsigned int), st), "memset");
     if (f.mode == B200RT_BACKPROJECT_DETERMINISTIC)
       ck(cudaMemsetAsync(f.acc64.p, 0, sizeof(unsigned long long) * f.h->geo->image_size(), st), "memset");
-    else if (f.upad.p && b.family == B200RT_BATCH_KERNELS_PATHS)
-      ck(cudaMemsetAsync(f.upad.p, 0, sizeof(float) * f.upad.n, st), "memset");
+    else if (f.usums.p && b.family == B200RT_BATCH_KERNELS_PATHS)
+      ck(cudaMemsetAsync(f.usums.p, 0, sizeof(float) * f.usums.n, st), "memset");
     else
       ck(cudaMemsetAsync(f.u.p, 0, sizeof(float) * f.h->geo->image_size(), st), "memset");
   }
@@ -522,12 +525,13 @@ void batch_subiteration(b200rt_batch& b, int k, cudaStream_t st) {
   for (auto& fp : b.frames)  // deterministic frames: their fixed-point numerators to float
     if (k <= fp->num_subiters && fp->mode == B200RT_BACKPROJECT_DETERMINISTIC)
       ck(launch_fixed_to_float(fp->acc64.p, fp->fixed_scale.p, fp->u.p, fp->h->geo->image_size(), st), "numerator");
-  if (b.family == B200RT_BATCH_KERNELS_PATHS)  // numerators in padded columns to the image's
+  if (b.family == B200RT_BATCH_KERNELS_PATHS)  // the numerators' sums to the image
     for (auto& fp : b.frames)
-      if (k <= fp->num_subiters && fp->upad.p) {
+      if (k <= fp->num_subiters && fp->usums.p) {
         const auto& d = fp->h->geo->desc();
-        ck(b200::launch_unpad_image(fp->upad.p, 0, fp->u.p, 0, static_cast<int64_t>(d.ny) * d.nx, d.nz,
-                                    b200::z_stride(fp->h->zparams), 1, st),
+        const b200::ZParams& z = fp->h->zparams;
+        ck(b200::launch_collect_images(fp->usums.p, 0, z.copies, fp->u.p, 0, static_cast<int64_t>(d.ny) * d.nx, d.nz,
+                                       z.planes > 1 ? b200::z_stride(z) : d.nz, 1, st),
            "numerator");
       }
   // every frame's update (OSMAPOSLReconstruction.cxx:394-510) in three launches

@@ -196,14 +196,21 @@ int b200rt_back_project(b200rt_projector* h, const float* projdata_host, float* 
            "H2D");
         ck(cudaEventRecord(h->copy_events[gi], h->copy_stream), "cudaEventRecord");
       }
-      ck(cudaMemsetAsync(h->st_img_b.p, 0, sizeof(float) * g.image_size(), st), "memset");
+      BackSums sums(*h, vg.off.back(), 1, st);
+      if (sums.own())
+        sums.clear(1);
+      else
+        ck(cudaMemsetAsync(h->st_img_b.p, 0, sizeof(float) * g.image_size(), st), "memset");
       for (size_t gi = 0; gi < G; ++gi) {
         ck(cudaStreamWaitEvent(st, h->copy_events[gi], 0), "cudaStreamWaitEvent");
         ck(projdata_layout_views(*h, h->st_pd_a.p, h->st_pd_b.p, true, vg.v0[gi], vg.v0[gi + 1], st), "layout");
         const int n = vg.off[gi + 1] - vg.off[gi];
-        if (n > 0)
+        if (sums.own())
+          sums.add(vg.list->p + vg.off[gi], n, h->st_pd_b.p, 0, 1, 0);
+        else
           add_back_paths(*h, vg.list->p + vg.off[gi], n, h->st_pd_b.p, 0, h->st_img_b.p, 0, 1, st, 0);
       }
+      if (sums.own()) sums.collect(h->st_img_b.p, 0, 1);
     } else {
       ck(cudaMemcpyAsync(h->st_pd_a.p, projdata_host, sizeof(float) * g.projdata_size(), cudaMemcpyHostToDevice, st),
          "H2D");

@@ -4,6 +4,16 @@
 
 using namespace b200;
 
+namespace {
+
+size_t most_groups(const std::vector<ZPath>& paths) {
+  size_t most = 1;
+  for (const ZPath& p : paths) most = std::max(most, p.recs.size());
+  return most;
+}
+
+}  // namespace
+
 namespace capi {
 
 // The chains and records of every path (zframe.hpp).  Returns false, leaving no tables, where the z-frame kernels do not
@@ -136,7 +146,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
               ZItemDev it{};
               it.rec0 = rec0;
               it.nrec = static_cast<int>(G.recs[gr].size());
-              it.flags = T;
+              it.flags = T | static_cast<int>((gr + ti + vi) & 3u) << kZTurn;
               it.path = path0[vi * ntangs + ti] + static_cast<int>(gr);
               int out = 0, nl = 0, ov = -2;
               for (int s = 0; s < 2 * kZChains; ++s) {
@@ -247,6 +257,8 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   ck(cudaStreamSynchronize(h.stream), "path tables");
   int64_t ngrp = 0;
   for (const ZPath& G : groups) ngrp += static_cast<int64_t>(G.recs.size());
+  const size_t ng_most = most_groups(groups);
+  z.copies = ng_most == 1 ? 1 : ng_most <= 3 ? 2 : 4;
   z.mean_rec = static_cast<int>(nrecs / std::max<int64_t>(1, ngrp));
   z.recs = h.z_recs.p;
   z.items = h.z_items.p;
@@ -352,16 +364,19 @@ bool pad_back(const b200rt_projector& h, int n, int batch) {
 
 namespace {
 
-// device memory of one call, given back to the handle's pool in stream order
-struct PoolBuf {
+// device memory of one call (given back to the handle's pool in stream order), or null: the kernels then take the plain image
+float* pool_alloc(b200rt_projector& h, size_t n, cudaStream_t st) {
   float* p = nullptr;
-  cudaStream_t st;
-  PoolBuf(b200rt_projector& h, size_t n, cudaStream_t s) : st(s) {
-    if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), n * sizeof(float), h.z_pool, st) != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;  // the kernels also take the plain image, more slowly
-    }
+  if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), n * sizeof(float), h.z_pool, st) != cudaSuccess) {
+    cudaGetLastError();
+    p = nullptr;
   }
+  return p;
+}
+struct PoolBuf {
+  float* p;
+  cudaStream_t st;
+  PoolBuf(b200rt_projector& h, size_t n, cudaStream_t s) : p(pool_alloc(h, n, s)), st(s) {}
   PoolBuf(const PoolBuf&) = delete;
   ~PoolBuf() {
     if (p) cudaFreeAsync(p, st);
@@ -411,29 +426,50 @@ void forward_paths(b200rt_projector& h, const int* list, int n, const float* ima
   }
 }
 
+// Memory of the call's own where its reductions go to padded columns or to several images, which collect() adds up.
+// images: at a time.
+BackSums::BackSums(b200rt_projector& h, int n, int images, cudaStream_t st) : h_(h), st_(st) {
+  if (!h.use_z || n <= 0) return;
+  const ZParams& z = h.zparams;
+  const bool padded = pad_back(h, n, images);
+  if (!padded && z.copies == 1) return;
+  const int64_t ncols = static_cast<int64_t>(h.params.ny) * h.params.nx;
+  stride_ = padded ? z_stride(z) : h.params.nz;
+  per_ = z_image_floats(ncols, stride_) * z.copies;
+  step_ = static_cast<int>(std::min<int64_t>(images, std::max<int64_t>(1, static_cast<int64_t>(kPadLimit) / per_)));
+  sums_ = pool_alloc(h, static_cast<size_t>(per_) * step_, st);
+}
+BackSums::~BackSums() {
+  if (sums_) cudaFreeAsync(sums_, st_);
+}
+void BackSums::clear(int images) {
+  ck(cudaMemsetAsync(sums_, 0, sizeof(float) * per_ * images, st_), "memset");
+}
+void BackSums::add(const int* list, int n, const float* pd, int64_t pd_stride, int images, int zero_ends) {
+  if (n > 0)
+    ck(launch_back_z(h_.params, h_.zparams, list, n, z_back_parts(h_, n), pd, pd_stride, sums_, per_, h_.zparams.copies,
+                     stride_ != h_.params.nz, images, st_, zero_ends),
+       "back projection");
+}
+void BackSums::collect(float* images, int64_t img_stride, int n) {
+  ck(launch_collect_images(sums_, per_, h_.zparams.copies, images, img_stride,
+                           static_cast<int64_t>(h_.params.ny) * h_.params.nx, h_.params.nz, stride_, n, st_),
+     "image sums");
+}
+
 // image b (overwritten) = the back projection of the list's items from projection data b
 void back_paths(b200rt_projector& h, const int* list, int n, const float* pd, int64_t pd_stride, float* images,
                 int64_t img_stride, int batch, cudaStream_t st, int zero_ends) {
   const int64_t ni = h.geo->image_size();
-  if (h.use_z && n > 0 && pad_back(h, n, batch)) {
-    const ZParams& z = h.zparams;
-    const int parts = z_back_parts(h, n);
-    const int64_t ncols = static_cast<int64_t>(h.params.ny) * h.params.nx, per = ncols * z_stride(z);
-    const int step =
-        static_cast<int>(std::min<int64_t>(batch, std::max<int64_t>(1, static_cast<int64_t>(kPadLimit) / per)));
-    PoolBuf pad(h, static_cast<size_t>(per) * step, st);
-    if (pad.p) {
-      for (int b = 0; b < batch; b += step) {
-        const int nb = std::min(step, batch - b);
-        ck(cudaMemsetAsync(pad.p, 0, sizeof(float) * per * nb, st), "memset");
-        ck(launch_back_z(h.params, z, list, n, parts, pd ? pd + b * pd_stride : nullptr, pd_stride, pad.p, per, 1, nb, st,
-                         zero_ends),
-           "back projection");
-        ck(launch_unpad_image(pad.p, per, images + b * img_stride, img_stride, ncols, h.params.nz, z_stride(z), nb, st),
-           "image planes");
-      }
-      return;
+  BackSums sums(h, n, batch, st);
+  if (sums.own()) {
+    for (int b = 0; b < batch; b += sums.step()) {
+      const int nb = std::min(sums.step(), batch - b);
+      sums.clear(nb);
+      sums.add(list, n, pd ? pd + b * pd_stride : nullptr, pd_stride, nb, zero_ends);
+      sums.collect(images + b * img_stride, img_stride, nb);
     }
+    return;
   }
   for (int b = 0; b < batch; ++b) ck(cudaMemsetAsync(images + b * img_stride, 0, sizeof(float) * ni, st), "memset");
   add_back_paths(h, list, n, pd, pd_stride, images, img_stride, batch, st, zero_ends);
@@ -444,7 +480,8 @@ void add_back_paths(b200rt_projector& h, const int* list, int n, const float* pd
                     int64_t img_stride, int batch, cudaStream_t st, int zero_ends) {
   if (n <= 0) return;
   if (h.use_z)
-    ck(launch_back_z(h.params, h.zparams, list, n, z_back_parts(h, n), pd, pd_stride, images, img_stride, 0, batch, st, zero_ends),
+    ck(launch_back_z(h.params, h.zparams, list, n, z_back_parts(h, n), pd, pd_stride, images, img_stride, 1, 0, batch, st,
+                     zero_ends),
        "back projection");
   else
     ck(launch_back_paths_atomic_batch(h.params, h.pparams, list, n, pd, pd_stride, images, img_stride, batch, st, zero_ends),

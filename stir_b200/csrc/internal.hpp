@@ -134,9 +134,10 @@ struct BatchFrameDev {
   // deterministic back projection of this frame: 64-bit fixed-point sums and their scale (null: float atomics)
   unsigned long long* acc64;
   const double* fixed_scale;
-  // z-frame geometries with several planes per lane: the estimate and the numerator in padded columns
+  // z-frame geometries with several planes per lane: the estimate in padded columns; and the numerator's sums, in padded
+  // columns or several images (ZParams::copies)
   const float* xpad;
-  float* upad;
+  float* usums;
 };
 struct BatchItem {
   int frame;

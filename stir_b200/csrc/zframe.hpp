@@ -28,11 +28,12 @@ struct __align__(16) ZRec {
 };
 static_assert(sizeof(ZRec) == 112, "a record is seven 16-byte pieces");
 constexpr uint32_t kZGuard = 1u << 12;
+constexpr int kZTurn = 8;
 
 // slot 2 m: the line of chain m whose planes grow with the basic row's, slot 2 m + 1: the z-reflected one
 struct ZItemDev {
   int rec0, nrec;       // the path group's records (nrec a multiple of 4)
-  int flags;            // T: bit 0 swap x/y, bit 1 negate x, bit 2 negate y
+  int flags;            // T: bit 0 swap x/y, bit 1 negate x, bit 2 negate y; from bit kZTurn on: the item's turn (ZParams::copies)
   int path;             // the path group's planes (ZParams::sixteenths)
   int2 slot[2 * kZChains];         // (index into lines[], basic bin) or (-1, -1)
   int16_t boff[2 * kZChains];      // back projection: the slot's datum 0 in the item's shared buffer (max_back floats)
@@ -53,6 +54,10 @@ struct ZParams {
   int nm;         // chains per item the kernels are compiled for: 4 or 6
   int planes;     // planes per lane: 1, 2 or 4 (32 x planes >= nz)
   int mean_rec;   // mean records of a path's groups
+  // images that the back projection's sums are spread over (1, 2 or 4), added at the end.  A path's chain groups add to a voxel
+  // one by one, where the column-staged kernels added their sum, so a voxel's float sum has as many times the terms and sqrt
+  // of that times the rounding error.  Spread over c images it has 1 / c of it: 2 images for up to 3 groups, 4 beyond.
+  int copies;
   int max_out;    // most projection values of one item
   int max_back;   // longest shared buffer of an item's data with the zeros around them
 };
@@ -76,22 +81,28 @@ inline ZSplit z_batch_split(ZSplit sp) {
 int z_forward_smem(const ZParams& z, int buffers);
 int z_resident_warps(const ZParams& z, bool forward);
 
+// floats of an image of columns `stride` apart, in whole 16-byte pieces: how far the images that take the items in turn are apart
+__host__ __device__ inline int64_t z_image_floats(int64_t ncols, int stride) { return (ncols * stride + 3) & ~int64_t(3); }
+
 // column stride (floats) of the padded images the kernels use when planes > 1
 inline int z_stride(const ZParams& z) { return 32 * z.planes; }
 
-// image [col][nz] <-> padded [col][stride] (planes past nz are zeros), `batch` images at the given strides
+// image [col][nz] -> padded [col][stride] (planes past nz are zeros), `batch` images at the given strides
 cudaError_t launch_pad_image(const float* in, int64_t in_stride, float* out, int64_t out_stride, int64_t ncols, int nz,
                              int stride, int batch, cudaStream_t st);
-cudaError_t launch_unpad_image(const float* in, int64_t in_stride, float* out, int64_t out_stride, int64_t ncols, int nz,
-                               int stride, int batch, cudaStream_t st);
+// image = the sum of `copies` images of columns `stride` apart (nz, or padded) that stand behind one another
+cudaError_t launch_collect_images(const float* in, int64_t in_stride, int copies, float* out, int64_t out_stride,
+                                  int64_t ncols, int nz, int stride, int batch, cudaStream_t st);
 
 // padded != 0: image has column stride z_stride(z) (16-byte aligned), else nz; the forward projection takes padded images
 // with sp.parts = 1 only
 cudaError_t launch_forward_z(const ProjParams& p, const ZParams& z, const int* list, int n, ZSplit sp, const float* image,
                              int64_t img_stride, int padded, float* out, int64_t out_stride, int batch, cudaStream_t st,
                              const FwdEpilogue* ep);
-cudaError_t launch_back_z(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* pd, int64_t pd_stride,
-                          float* image, int64_t img_stride, int padded, int batch, cudaStream_t st, int zero_ends);
+// copies: images behind one another that take the items in turn (1: the image itself)
+cudaError_t launch_back_z(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* pd,
+                          int64_t pd_stride, float* image, int64_t img_stride, int copies, int padded, int batch,
+                          cudaStream_t st, int zero_ends);
 cudaError_t launch_back_z_fixed(const ProjParams& p, const ZParams& z, const int* list, int n, int parts, const float* pd,
                                 unsigned long long* acc, const double* scale, cudaStream_t st, int zero_ends);
 

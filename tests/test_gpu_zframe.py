@@ -195,3 +195,21 @@ def test_forward_sums_are_short(cuda_device):
         first += pdi.num_views * ntang * nax
     error = np.linalg.norm(np.array(mine) - np.array(exact)) / np.linalg.norm(exact)
     assert error <= 1.5 * 2.0 ** -24, error
+
+
+@pytest.mark.parametrize("rays,span", [(1, 1), (2, 3)])
+def test_back_sums_are_short(rays, span, cuda_device):
+    """The rounding of a voxel's float sum where a path's rows fall into several groups of chains, against the fixed-point sums
+    (whose own error is below 3e-8).  Adding N values of one size rounds N times, by 0.3 of 2^-23 of the running value: 0.3
+    2^-23 sqrt(N / 3) of the sum (2-norm over the voxels).  One addition a view and column crossed makes N = 1.3 x the views;
+    one a group two to three times as many."""
+    import torch
+    from stir_b200.projectors import RayTracingProjector
+    sc = G.Scanner(8, 288, 300.0, 0.0, 4.0, float(np.float32(np.pi * 300.0 / 288)))
+    proj = RayTracingProjector(G.ProjDataInfoCTI(sc, span, 7, 144, 64), G.ImageGeometry(15, 64, 64, (2.0, 4.0, 4.0)),
+                               num_tangential_LORs=rays, device=cuda_device)
+    y = torch.rand(proj.projdata_size, device="cuda", generator=torch.Generator("cuda").manual_seed(11))
+    exact = proj.back_dev(y, mode=_abi.BACKPROJECT_DETERMINISTIC).double()
+    got = proj.back_dev(y).double()
+    error = float((got - exact).norm() / exact.norm())
+    assert error <= 0.3 * 2.0 ** -23 * (1.3 * 144 / 3) ** 0.5, error
