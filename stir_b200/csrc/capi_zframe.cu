@@ -6,6 +6,8 @@ using namespace b200;
 
 namespace {
 
+constexpr size_t kPadLimit = size_t(1) << 26;  // floats of padded images or image sums at a time (256 MiB)
+
 size_t most_groups(const std::vector<ZPath>& paths) {
   size_t most = 1;
   for (const ZPath& p : paths) most = std::max(most, p.recs.size());
@@ -272,14 +274,15 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   h.h_path_items = std::move(path_items);
   h.paths_view_split =
       std::find(h.h_item_out_view.begin(), h.h_item_out_view.end(), -1) == h.h_item_out_view.end();
-  // padded images come from a pool of the handle's own, in stream order: calls on several streams or threads have their
-  // own, freed memory stays with the handle until it is destroyed
+  // padded images and image sums come from a pool of the handle's own, in stream order: calls on several streams or threads
+  // have their own.  The pool keeps what one call needs (kPadLimit, or one image's where that is more); what calls side by
+  // side had beyond that goes back to the device at the next synchronisation, and all of it with the handle.
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
   props.location.id = h.device;
   ck(cudaMemPoolCreate(&h.z_pool, &props), "cudaMemPoolCreate");
-  uint64_t keep = UINT64_MAX;
+  uint64_t keep = sizeof(float) * std::max<uint64_t>(kPadLimit, static_cast<uint64_t>(padded) * z.copies);
   ck(cudaMemPoolSetAttribute(h.z_pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
   h.use_paths = h.use_z = true;
   return true;
@@ -364,8 +367,12 @@ bool pad_back(const b200rt_projector& h, int n, int batch) {
 
 namespace {
 
-// device memory of one call (given back to the handle's pool in stream order), or null: the kernels then take the plain image
+// Device memory of one call (given back to the handle's pool in stream order), or null: the kernels then take the plain image.
+// None while the stream is captured: allocation nodes would keep a graph from being instantiated twice, cloned or a child.
 float* pool_alloc(b200rt_projector& h, size_t n, cudaStream_t st) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) cudaGetLastError();
+  if (capturing != cudaStreamCaptureStatusNone) return nullptr;
   float* p = nullptr;
   if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), n * sizeof(float), h.z_pool, st) != cudaSuccess) {
     cudaGetLastError();
@@ -382,8 +389,6 @@ struct PoolBuf {
     if (p) cudaFreeAsync(p, st);
   }
 };
-
-constexpr size_t kPadLimit = size_t(1) << 28;  // floats of padded images at a time (1 GiB)
 
 }  // namespace
 

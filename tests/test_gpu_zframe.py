@@ -213,3 +213,47 @@ def test_back_sums_are_short(rays, span, cuda_device):
     got = proj.back_dev(y).double()
     error = float((got - exact).norm() / exact.norm())
     assert error <= 0.3 * 2.0 ** -23 * (1.3 * 144 / 3) ** 0.5, error
+
+
+@pytest.mark.parametrize("case", ["padded images", "image sums"])
+def test_captured_calls(case, cuda_device):
+    """Calls captured into a graph allocate nothing: the graph can be instantiated twice, which allocation nodes forbid."""
+    import torch
+    from stir_b200.projectors import RayTracingProjector
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    if case == "padded images":  # 109 of 128 planes, 1.5 million columns walked
+        sc = G.Scanner(55, 192, 200.0, 0.0, 4.0, float(np.float32(np.pi * 200.0 / 192)))
+        pdi, img = G.ProjDataInfoCTI(sc, 11, 30, 96, 101), G.ImageGeometry(109, 71, 71, (2.0, 4.0, 4.0))
+    else:  # three chain groups
+        sc = G.Scanner(8, 96, 100.0, 0.0, 4.0, float(np.float32(np.pi * 100.0 / 96)))
+        pdi, img = G.ProjDataInfoCTI(sc, 1, 7, 48, 40), G.ImageGeometry(15, 40, 40, (2.0, 4.0, 4.0))
+    proj = RayTracingProjector(pdi, img, device=cuda_device)
+    gen = torch.Generator("cuda").manual_seed(12)
+    x = torch.rand(proj.device_image_shape, device="cuda", generator=gen)
+    y = torch.rand(proj.projdata_size, device="cuda", generator=gen)
+    want = proj.forward_dev(x), proj.back_dev(y)
+    out, back = proj.empty_projdata(), proj.empty_image()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess, r[0]
+        return r[1] if len(r) == 2 else None
+
+    ok(rt.cudaStreamBeginCapture(stream.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal))
+    proj.forward_dev(x, out=out, stream=stream)
+    proj.back_dev(y, out=back, stream=stream)
+    graph = ok(rt.cudaStreamEndCapture(stream.cuda_stream))
+    execs = [ok(rt.cudaGraphInstantiate(graph, 0)) for _ in range(2)]
+    for e in execs:
+        out.zero_()
+        back.zero_()
+        torch.cuda.synchronize()
+        ok(rt.cudaGraphLaunch(e, stream.cuda_stream))
+        stream.synchronize()
+        assert torch.equal(out, want[0])
+        # two float sums of a voxel in another order: at most 1.3 x 96 views x 3 groups of one size each
+        assert float((back - want[1]).norm() / want[1].norm()) <= 2 * 0.3 * 2.0 ** -23 * (1.3 * 96) ** 0.5
+    for e in execs:
+        ok(rt.cudaGraphExecDestroy(e))
+    ok(rt.cudaGraphDestroy(graph))
