@@ -70,9 +70,11 @@ struct b200rt_batch {
   // item lists by (order, subset of each frame or -1)
   std::map<std::vector<int>, std::unique_ptr<DevBuf<b200::BatchItem>>> items;
   std::map<std::vector<int>, int> item_counts;
-  // the path-item family's lists, kernel by kernel: (entry of path_kernels, first item, items)
+  // the path-item family's lists, kernel by kernel: (entry of path_kernels, whether warps share the items, first item, items)
   struct Part {
-    int kernel, first, count;
+    int kernel;
+    bool shared;
+    int first, count;
   };
   std::map<std::vector<int>, std::vector<Part>> item_parts;
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
@@ -245,7 +247,7 @@ void batch_finalize(b200rt_batch& b) {
     fd.push_back(d);
   }
   b.d_frames.upload(fd, st);
-  b.counters.alloc(2 * std::max<size_t>(1, b.path_kernels.size()));  // per kernel and direction
+  b.counters.alloc(4 * std::max<size_t>(1, b.path_kernels.size()));  // per kernel, direction and whether items are shared
   ck(cudaDeviceGetAttribute(&b.num_sms, cudaDevAttrMultiProcessorCount, b.device), "device attribute");
   if (b.avail[B200RT_BATCH_KERNELS_PATHS]) {
     int most[2] = {0, 0};
@@ -347,7 +349,7 @@ const BatchItem* batch_items(b200rt_batch& b, int k, int order, int& count) {
       for (int q = 0; q < parts; ++q) entries[fi].push_back(BatchItem{code, bin});
     if (zf) {
       unit[fi] = b200::kZWarps;
-      while (entries[fi].size() % b200::kZWarps) entries[fi].push_back(BatchItem{frame, -1});
+      while (entries[fi].size() % b200::kZWarps) entries[fi].push_back(BatchItem{code, -1});
     }
   }
   if (order == 2) {
@@ -373,11 +375,17 @@ const BatchItem* batch_items(b200rt_batch& b, int k, int order, int& count) {
   if (b.family == B200RT_BATCH_KERNELS_PATHS) {  // kernel by kernel, in the order above within each
     std::vector<BatchItem> by;
     std::vector<b200rt_batch::Part> parts;
-    for (size_t k = 0; k < b.path_kernels.size(); ++k) {
+    auto take = [&](int k, bool shared) {
       const int first = static_cast<int>(by.size());
       for (const BatchItem& it : list)
-        if (b.geom_kernel[b.frames[it.frame & ((1 << b200::kZFrameBits) - 1)]->geom] == static_cast<int>(k)) by.push_back(it);
-      parts.push_back({static_cast<int>(k), first, static_cast<int>(by.size()) - first});
+        if (b.geom_kernel[b.frames[b200::z_frame_of(it.frame)]->geom] == k && (b200::z_split_of(it.frame).parts > 1) == shared)
+          by.push_back(it);
+      if (static_cast<int>(by.size()) > first || !shared)
+        parts.push_back({k, shared, first, static_cast<int>(by.size()) - first});
+    };
+    for (size_t k = 0; k < b.path_kernels.size(); ++k) {
+      take(static_cast<int>(k), false);
+      take(static_cast<int>(k), true);
     }
     list.swap(by);
     b.item_parts[key] = std::move(parts);
@@ -446,11 +454,11 @@ cudaError_t batch_launch(b200rt_batch& b, int dir, int k, int order, const Batch
     for (const auto& part : b.item_parts.at(item_key(b, k, order))) {
       const auto& pk = b.path_kernels[part.kernel];
       const int g = std::min(grid, pk.max_ctas[dir] * b.num_sms);
-      unsigned* counter = b.counters.p + 2 * part.kernel + dir;
+      unsigned* counter = b.counters.p + 4 * part.kernel + 2 * part.shared + dir;
       const BatchItem* it = items + part.first;
       cudaError_t e;
       if (pk.z >= 0)
-        e = b200::launch_z_batch(b.geoms[pk.z]->zparams, dir == 0, b.d_geoms.p, b.d_zgeoms.p, b.d_frames.p, it,
+        e = b200::launch_z_batch(b.geoms[pk.z]->zparams, dir == 0, part.shared, b.d_geoms.p, b.d_zgeoms.p, b.d_frames.p, it,
                                  part.count / b200::kZWarps, counter, pk.smem[dir], g, st);
       else if (dir == 0)
         e = b200::launch_forward_batch_paths(b.d_geoms.p, b.d_pgeoms.p, b.npa, pk.smem[0], b.d_frames.p, it, part.count,

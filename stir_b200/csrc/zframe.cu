@@ -843,7 +843,8 @@ __device__ __forceinline__ int next_z_unit(unsigned* counter, int nunits) {
   return s_unit < nunits ? s_unit : -1;
 }
 
-template <int NM, int P>
+// (SHARED: see forward_z_item; an instance of its own, as one kernel with both forms ran out of registers)
+template <int NM, int P, bool SHARED>
 __global__ void __launch_bounds__(kZWarps * 32, forward_ctas(NM, P))
     forward_z_batch_kernel(const ProjParams* __restrict__ geoms, const ZParams* __restrict__ zgeoms,
                            const BatchFrameDev* __restrict__ frames, const BatchItem* __restrict__ items, int nunits,
@@ -860,12 +861,8 @@ __global__ void __launch_bounds__(kZWarps * 32, forward_ctas(NM, P))
     constexpr bool kPad = P > 1;
     const ZSplit sp = z_split_of(wi.frame);
     const float* x = kPad ? f.xpad : f.x;
-    if (sp.parts > 1)
-      forward_z_item<NM, P, kPad, true>(geoms[f.geom], z, z.items[wi.bin], sp, smem + warp * warp_smem, warp_smem, x, f.ratio,
+    forward_z_item<NM, P, kPad, SHARED>(geoms[f.geom], z, z.items[wi.bin], sp, smem + warp * warp_smem, warp_smem, x, f.ratio,
                                         f.ep, ll, ncancel, warp, lane);
-    else
-      forward_z_item<NM, P, kPad, false>(geoms[f.geom], z, z.items[wi.bin], sp, smem + warp * warp_smem, warp_smem, x, f.ratio,
-                                         f.ep, ll, ncancel, warp, lane);
     for (int o = 16; o > 0; o >>= 1) ncancel += __shfl_xor_sync(kFull, ncancel, o);
     if (lane == 0 && ncancel && f.ep.cancelled) atomicAdd(f.ep.cancelled, ncancel);
   }
@@ -1084,7 +1081,7 @@ int z_batch_smem(const ZParams& z, bool forward, int buffers) {
   return kZWarps * (forward ? forward_smem(z, buffers) : back_smem(z));
 }
 
-cudaError_t launch_z_batch(const ZParams& z, bool forward, const ProjParams* geoms, const ZParams* zgeoms,
+cudaError_t launch_z_batch(const ZParams& z, bool forward, bool shared, const ProjParams* geoms, const ZParams* zgeoms,
                            const BatchFrameDev* frames, const BatchItem* items, int nunits, unsigned* counter, int smem,
                            int grid, cudaStream_t st) {
   if (nunits <= 0) return cudaSuccess;
@@ -1097,8 +1094,10 @@ cudaError_t launch_z_batch(const ZParams& z, bool forward, const ProjParams* geo
     kernel<<<grid, kZWarps * 32, smem, st>>>(geoms, zgeoms, frames, items, nunits, counter, smem / kZWarps);
     return cudaGetLastError();
   };
-  return forward ? z_variant(z, [&]<int NM, int P>() { return run(forward_z_batch_kernel<NM, P>); })
-                 : z_variant(z, [&]<int NM, int P>() { return run(back_z_batch_kernel<NM, P>); });
+  return z_variant(z, [&]<int NM, int P>() {
+    if (!forward) return run(back_z_batch_kernel<NM, P>);
+    return shared ? run(forward_z_batch_kernel<NM, P, true>) : run(forward_z_batch_kernel<NM, P, false>);
+  });
 }
 
 int z_batch_max_ctas_per_sm(const ZParams& z, bool forward, int smem) {
@@ -1111,7 +1110,7 @@ int z_batch_max_ctas_per_sm(const ZParams& z, bool forward, int smem) {
     }
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kZWarps * 32, smem);
   };
-  const cudaError_t e = forward ? z_variant(z, [&]<int NM, int P>() { return count(forward_z_batch_kernel<NM, P>); })
+  const cudaError_t e = forward ? z_variant(z, [&]<int NM, int P>() { return count(forward_z_batch_kernel<NM, P, false>); })
                                 : z_variant(z, [&]<int NM, int P>() { return count(back_z_batch_kernel<NM, P>); });
   return e == cudaSuccess ? n : 0;
 }

@@ -127,7 +127,8 @@ inline int z_frame_split(int frame, ZSplit sp) {
 }
 int z_batch_smem(const ZParams& z, bool forward, int buffers);
 int z_batch_max_ctas_per_sm(const ZParams& z, bool forward, int smem);
-cudaError_t launch_z_batch(const ZParams& z, bool forward, const ProjParams* geoms, const ZParams* zgeoms,
+// shared: the units hold items that warps share (forward: a kernel of its own)
+cudaError_t launch_z_batch(const ZParams& z, bool forward, bool shared, const ProjParams* geoms, const ZParams* zgeoms,
                            const BatchFrameDev* frames, const BatchItem* items, int nunits, unsigned* counter, int smem,
                            int grid, cudaStream_t st);
 
