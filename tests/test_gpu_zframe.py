@@ -48,11 +48,13 @@ def case(request, cuda_device):
 
 
 def _bound(orc):
-    """Relative error of a float sum of n non-negative products, each side at most n roundings of 2^-24; n: the longest
-    row, and for a voxel the lines through it (fewer than 4 per view and ring pair at these sizes)."""
+    """Relative error of a float sum of n non-negative products against another order of the same sum: each of the n additions
+    rounds by at most half a unit (2^-24 of the running value), with either sign, 0.6 of that on average; 6 standard deviations
+    of both sides' sum.  n: the longest row (up to 3 planes a column), and for a voxel the lines through it: two tangential
+    positions a view, and up to four axial positions of each segment within a plane of it."""
     g = orc.geometry
-    n = 4 * max(g.nx, g.ny) * 3 + 4 * g.num_views * g.num_rings
-    return 2 * n * 2.0 ** -24
+    n = max(3 * (g.nx + g.ny), 2 * 4 * g.num_views * (2 * g.max_segment_num + 1))
+    return 6 * 0.6 * 2.0 ** -24 * (2 * n) ** 0.5
 
 
 @pytest.mark.parametrize("subset", [(0, 1), (1, 4)])
@@ -162,6 +164,42 @@ def test_items_shared_by_warps(name, cuda_device):
                                                             subset_num=1, num_subsets=nsub)).cpu().numpy()
     ref = orc.forward(x, 1, nsub)
     assert not np.isnan(got).any() and np.array_equal(np.isinf(got), np.isinf(ref))
+
+
+@pytest.mark.parametrize("name", ["1 plane a lane", "1 plane, span 1", "2 planes, two rays", "4 planes"])
+def test_batched_frames_of_shared_items(name, cuda_device):
+    """Batched deterministic frames whose items are shared by warps equal their own reconstructions bit for bit, and float ones
+    up to the rounding of the back projection's sums."""
+    import torch
+    from stir_b200.batch import BatchedOSMAPOSL
+    from stir_b200.osmaposl import OSMAPOSLReconstruction
+    from stir_b200.projectors import RayTracingProjector
+    (pdi, img, rays), _ = SHARED[name]
+    proj = RayTracingProjector(pdi, img, num_tangential_LORs=rays, device=cuda_device)
+    gen = torch.Generator("cuda").manual_seed(13)
+    x0 = torch.rand(proj.device_image_shape, device="cuda", generator=gen) + 0.5
+    y = proj.forward_dev(x0) * (0.5 + torch.rand(proj.projdata_size, device="cuda", generator=gen))
+    add = torch.full_like(y, float(y.mean()))
+    for mode in (_abi.BACKPROJECT_DETERMINISTIC, _abi.BACKPROJECT_ATOMIC):
+        def recon(n):
+            return OSMAPOSLReconstruction(proj, y, additive=add, num_subsets=6, num_subiterations=n, back_projection_mode=mode)
+        own, ref = recon(4).set_up(), proj.empty_image().fill_(1.0)
+        own.reconstruct(ref)
+        batch, xs = BatchedOSMAPOSL(), []
+        for n in (4, 4, 2):
+            r = recon(n)
+            r.sensitivities = own.sensitivities
+            xs.append(proj.empty_image().fill_(1.0))
+            batch.add(r, xs[-1])
+        batch.set_config(kernels=_abi.BATCH_KERNELS_PATHS)
+        batch.reconstruct()
+        torch.cuda.synchronize()
+        batch.close()
+        for x in xs[:2]:
+            if mode == _abi.BACKPROJECT_DETERMINISTIC:
+                assert torch.equal(x, ref)
+            else:
+                assert float((x - ref).norm() / ref.norm()) <= 4 * 1e-6  # four steps of at most 1e-6 each
 
 
 def test_forward_sums_are_short(cuda_device):
