@@ -271,10 +271,6 @@ __host__ __device__ inline PathSmemBack path_smem_back(int nz, int max_lines, in
 }
 
 // launchers (paths.cu); the item lists hold indices into PathParams::items
-cudaError_t launch_forward_paths(const ProjParams& p, const PathParams& pp, const int* items, int nitems,
-                                 const float* image, float* projdata, cudaStream_t st, const FwdEpilogue* ep);
-cudaError_t launch_back_paths_atomic(const ProjParams& p, const PathParams& pp, const int* items, int nitems,
-                                     const float* projdata, float* image, cudaStream_t st, int zero_ends);
 cudaError_t launch_back_paths_fixed(const ProjParams& p, const PathParams& pp, const int* items, int nitems,
                                     const float* projdata, unsigned long long* acc, const double* scale,
                                     cudaStream_t st, int zero_ends);

@@ -944,11 +944,6 @@ cudaError_t launch_forward_paths_batch(const ProjParams& p, const PathParams& pp
   }
 }
 
-cudaError_t launch_forward_paths(const ProjParams& p, const PathParams& pp, const int* items, int nitems,
-                                 const float* image, float* projdata, cudaStream_t st, const FwdEpilogue* ep) {
-  return launch_forward_paths_batch(p, pp, items, nitems, image, 0, projdata, 0, 1, st, ep);
-}
-
 cudaError_t launch_forward_batch_paths(const ProjParams* geoms, const PathParams* pgeoms, int npa, int smem_bytes,
                                        const BatchFrameDev* frames, const BatchItem* items, int nitems, unsigned* counter,
                                        int grid, cudaStream_t st) {
@@ -980,11 +975,6 @@ int batch_paths_max_ctas_per_sm(int npa, int smem_bytes, bool forward) {
   int n = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kPathThreads, smem_bytes) != cudaSuccess) return 0;
   return n;
-}
-
-cudaError_t launch_back_paths_atomic(const ProjParams& p, const PathParams& pp, const int* items, int nitems,
-                                     const float* projdata, float* image, cudaStream_t st, int zero_ends) {
-  return launch_back_paths(p, pp, items, nitems, projdata, 0, FloatCols{image}, 0, 1, st, zero_ends);
 }
 
 cudaError_t launch_back_paths_atomic_batch(const ProjParams& p, const PathParams& pp, const int* items, int nitems,
