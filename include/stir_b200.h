@@ -197,7 +197,15 @@ int b200rt_set_viewgram(b200rt_projector* h, float* projdata_dev, int segment_nu
  * (src/include/stir/recon_buildblock/ForwardProjectorByBin.h:108): writes the
  * bins of the views in subset `subset_num` of `num_subsets`
  * (detail::find_basic_vs_nums_in_subset, find_basic_vs_nums_in_subset.cxx:32-70);
- * num_subsets=1 projects everything.  Bins of other subsets are left as they are. */
+ * num_subsets=1 projects everything.  Bins of other subsets are left as they are.
+ *
+ * Device memory of a call.  This and the other projecting entry points may take up to 256 MiB (or one image in
+ * padded columns or its sums, where that is more) from a stream-ordered pool of the projector: a copy of images of 33
+ * to 128 planes in padded columns, and the image that a back projection's sums are added up in.  The pool keeps that
+ * much, returns what calls side by side took beyond it at the next synchronisation, and all of it with
+ * b200rt_destroy; it is outside any caching allocator of the caller.  Where it cannot be had, and while `stream` is
+ * being captured, the call works on the plain image: nothing is allocated and no allocation node enters the graph;
+ * the same forward results, more slowly, and back projections whose sums may round up to twice as much. */
 int b200rt_forward_project_dev(b200rt_projector* h, const float* image_dev, float* projdata_dev,
                                int subset_num, int num_subsets, void* stream);
 
@@ -282,7 +290,7 @@ int b200rt_prior_value_dev(b200rt_projector* h, const b200rt_prior* prior, const
  * those views only (lines of other views are skipped, and path items without a line in the shard); summed over
  * shards that partition the views they give the whole data's result.  For the multi-GPU reconstruction that keeps
  * only its share of y, a and m on each GPU (the data partition of STIR's MPI build, distributed.cxx:161-225).
- * Needs the column-staged kernels (non-TOF data; B200RT_ERR_UNSUPPORTED otherwise).  Entry points that address the
+ * Needs the path-item kernels (non-TOF data; B200RT_ERR_UNSUPPORTED otherwise).  Entry points that address the
  * whole data (host buffers, layout conversions, viewgrams, streams, list mode, OSSPS, batches, the allocation-free
  * log-likelihood) return B200RT_ERR_STATE on a shard.  views = NULL or num_views = 0 restores the whole data. */
 int b200rt_set_view_shard(b200rt_projector* h, const int32_t* views, int num_views);
@@ -290,8 +298,9 @@ int b200rt_set_view_shard(b200rt_projector* h, const int32_t* views, int num_vie
 /* A batch of images through one projector (no STIR counterpart: STIR projects one image at a time; the batches of
  * torch.autograd and of noise realisations).  Image b is at images_dev + b*image_stride (device layout), its
  * projection data at projdata_dev + b*projdata_stride; strides in floats, at least an image / the projection data.
- * Where the column-staged kernels apply (non-TOF projectors) each call is one launch over (path item, image);
- * otherwise, and for the deterministic back projection, the images go one at a time.  Results equal the
+ * Where the path-item kernels apply (non-TOF projectors) each call is one launch over (path item, image), or one for
+ * every 256 MiB of padded images or image sums (b200rt_forward_project_dev); otherwise, and for the deterministic back
+ * projection, the images go one at a time.  Results equal the
  * single-image entry points' (the forward bit for bit; the atomic back projection to the order of float additions).
  * Replaces a loop over ForwardProjectorByBin::forward_project / BackProjectorByBin::back_project
  * (src/recon_buildblock/ForwardProjectorByBin.cxx:168-230, BackProjectorByBin.cxx:182-229). */
@@ -315,7 +324,7 @@ int b200rt_log_likelihood_batch_dev(b200rt_projector* h, const float* images_dev
  * ratio_dev + b * ratio_stride (device layout; bins outside the subset are not written), so that the gradient is then
  * one b200rt_back_project_batch_dev of the ratios, without projecting again.  No STIR counterpart: STIR computes
  * the value (accumulate_loglikelihood, ...AndProjData.cxx:1483-1515) and the sub-gradient (:1421-1481) in separate
- * passes.  Column-staged projectors only (B200RT_ERR_UNSUPPORTED otherwise).  Synchronises and writes values[b]. */
+ * passes.  Path-item projectors only (B200RT_ERR_UNSUPPORTED otherwise).  Synchronises and writes values[b]. */
 int b200rt_log_likelihood_and_ratio_batch_dev(b200rt_projector* h, const float* images_dev, int64_t image_stride,
                                                const float* y_dev, int64_t y_stride, const float* additive_dev,
                                                int64_t additive_stride, const float* mult_dev, int64_t mult_stride,
@@ -336,15 +345,18 @@ int b200rt_log_likelihood_gradient_batch_dev(b200rt_projector* h, const float* i
  * and view list are selected on the device from tables made by b200rt_create, and its scratch (those
  * lists, the viewgram thresholds and one FP64 partial sum per work item) lives in a fixed 2.02 MiB
  * array compiled into the library, which every GPU that loads the library holds until the process
- * exits.  It runs the same kernel on the same work items as b200rt_log_likelihood_dev (path items,
- * or basic bins with all their timing bins for a TOF projector), so the two agree to the last bit.
- *   - limits: at most 131072 work items in the subset (path items, or basic bins), 4096 views of the
+ * exits.  A projector whose path items the z-frame kernels cut into parts keeps the list and the partial sums of the
+ * parts itself (12 bytes a part, made by b200rt_create; 1 MB on a 64-ring, 504-detector scanner).  It runs the same
+ * sums on the same work items as b200rt_log_likelihood_dev (path items, or basic bins with all their timing bins for
+ * a TOF projector), so the two agree to the last bit; where that call copies the image to padded columns first, this
+ * one reads it as it is, more slowly.
+ *   - limits: at most 131072 work items in the subset (path items, however many parts, or basic bins), 4096 views of the
  *     subset, and 131072 viewgrams in the data (num_tof_bins * (2*max_segment_num+1) * num_views);
  *     larger requests return B200RT_ERR_TOO_LARGE with the counts in b200rt_last_error;
  *   - the result is written to out_dev, a device double the caller provides; the call is
  *     asynchronous on `stream` and does not synchronise;
- *   - all calls share the one array: calls that overlap on the GPU (other streams, other threads)
- *     race and corrupt each other's results;
+ *   - all calls share the one array (and those on one projector its list): calls that overlap on the GPU (other
+ *     streams, other threads) race and corrupt each other's results;
  *   - the first call on a device looks up the array's device address (cudaGetSymbolAddress) and
  *     keeps it for the life of the process; make that first call before any stream capture, and do
  *     not reset the device (cudaDeviceReset) between calls. */
@@ -419,8 +431,8 @@ int b200rt_back_project(b200rt_projector* h, const float* projdata_host, float* 
  * sensitivities, subset count and prior.  Batched sub-iteration k advances every frame with
  * num_subiterations >= k by its own sub-iteration k, subset (start_subset + k - 1) % num_subsets, with
  * the result of b200rt_osmaposl_subiteration_dev (atomic back projection) up to float rounding.  Per k:
- * one persistent forward launch (ratio epilogue) and one persistent back projection cover every
- * frame's subset, and the frames' updates run as three launches over all frames; the data thresholds of
+ * one persistent forward launch (ratio epilogue) and one persistent back projection for each kernel that the frames'
+ * projectors use cover every frame's subset, and the frames' updates run as three launches over all frames; the data thresholds of
  * divide_and_truncate are computed once per b200rt_batch_run call.  Projectors passed to
  * add_frame must outlive the batch and are not used concurrently by the caller while it runs. */
 typedef struct b200rt_batch b200rt_batch;
@@ -434,10 +446,11 @@ typedef struct {
 } b200rt_batch_config;
 /* Kernel families of the batched projectors (how the work of a frame is cut into work items):
  * AUTO: the first the frames allow of PATHS, TOF_GROUPED, PACKED, BASIC_BINS;
- * PATHS: one CTA per (frame, path item), the image columns of the path staged in shared memory, lanes on axial
- *   positions (every frame's projector has path tables; the only family for deterministic frames);
- * TOF_GROUPED: one warp per (frame, basic bin) with all its timing bins in registers, lanes on (line, axial
- *   position) (TOF frames with one timing-bin count);
+ * PATHS: (frame, path item) by the kernels of the frame's own projector: up to four warps an item, lanes on image planes
+ *   (z-frame kernels, images of at most 128 planes), or one CTA an item, the image columns of the path staged in shared
+ *   memory, lanes on axial positions (every frame's projector has path tables; the only family for deterministic frames);
+ * TOF_GROUPED: one warp per (frame, basic bin) with all its timing bins in registers, lanes on (group of timing bins, axial
+ *   position), or for longer lines and more timing bins on (line, axial position) (TOF frames with one timing-bin count);
  * PACKED: one warp per (frame, basic bin or TOF bin), lanes on (line, axial position) (at most 16 axial positions);
  * BASIC_BINS: one CTA per (frame, basic bin or TOF bin), one warp per related line, lanes on axial positions. */
 #define B200RT_BATCH_KERNELS_AUTO 0
@@ -458,7 +471,7 @@ int b200rt_batch_add_frame(b200rt_batch* b, b200rt_projector* h, float* estimate
 /* Back projection of a frame: B200RT_BACKPROJECT_ATOMIC (the default) or B200RT_BACKPROJECT_DETERMINISTIC, whose
  * numerator is the same 64-bit fixed-point sum as b200rt_osmaposl_subiteration_dev's in that mode (scale from the
  * ratio's bound 1e4), so the frame's reconstruction is bit-reproducible and equal to its own one-frame run.
- * Deterministic frames need the column-staged kernels (non-TOF projectors; B200RT_ERR_UNSUPPORTED otherwise). */
+ * Deterministic frames need the path-item kernels (non-TOF projectors; B200RT_ERR_UNSUPPORTED otherwise). */
 int b200rt_batch_set_frame_mode(b200rt_batch* b, int frame, int back_projection_mode);
 int b200rt_batch_num_frames(const b200rt_batch* b);
 /* Runs batched sub-iterations first..first+count-1 on `stream`.  use_graph != 0: the sequence is

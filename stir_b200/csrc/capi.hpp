@@ -146,12 +146,13 @@ struct b200rt_projector {
   DevBuf<ZPlanes> z_planes;
   ZParams zparams{};
   cudaMemPool_t z_pool = nullptr;  // padded images of calls in flight
+  std::vector<int> h_item_block;   // an item's block of kZWarps tangential positions
   std::vector<char> h_item_lead;   // the first of a path item's parts (groups of chains, further lines)
   DevBuf<int> z_work;              // the allocation-free log-likelihood's work list and partial sums
   DevBuf<double> z_partials;
   std::vector<int> h_item_view;  // basic view of each path item
   std::vector<PathItemDev> h_path_items;
-  std::map<std::pair<int, int>, std::unique_ptr<DevBuf<int>>> path_lists;
+  std::map<std::pair<int, int>, std::unique_ptr<DevBuf<int>>> path_lists, back_lists;  // (the latter where in another order)
   std::map<std::pair<int, int>, int> path_counts;
   // staging for the host API
   DevBuf<float> st_img_a, st_img_b, st_pd_a, st_pd_b;
@@ -198,7 +199,9 @@ int fail(b200rt_projector* h, int code, const std::string& msg);
 int status_of(const std::exception& e);
 void setup_projector(b200rt_projector& h);
 const int* subset_list(b200rt_projector& h, int subset, int nsub, int& count);
-const int* path_list(b200rt_projector& h, int subset, int nsub, int& count);
+// the path items of a subset, for the forward or the back projection (back_order)
+const int* path_list(b200rt_projector& h, int subset, int nsub, int& count, bool back = false);
+void back_order(const b200rt_projector& h, std::vector<int>& items);
 const int* tof_group_list(b200rt_projector& h, int subset, int nsub, int& count);
 void forward_subset(b200rt_projector& h, const float* image, float* out, int subset, int nsub, cudaStream_t st,
                     const FwdEpilogue* ep = nullptr);

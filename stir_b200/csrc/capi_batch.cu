@@ -307,6 +307,7 @@ const BatchItem* batch_items(b200rt_batch& b, int k, int order, int& count) {
     if (b.family == B200RT_BATCH_KERNELS_PATHS) {
       for (int i = 0; i < static_cast<int>(h.h_item_view.size()); ++i)
         if (h.h_item_view[i] % f.nsub == key[fi + 2]) bins.push_back(i);
+      back_order(h, bins);
       if (order == 1) {
         std::stable_sort(bins.begin(), bins.end(), [&](int a, int c) {
           const auto& pa = h.h_path_items[a];

@@ -71,7 +71,7 @@ int b200rt_back_project_batch_dev(b200rt_projector* h, const float* projdata_dev
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (h->use_paths && back_projection_mode == B200RT_BACKPROJECT_ATOMIC) {
       int n = 0;
-      const int* list = path_list(*h, subset_num, num_subsets, n);
+      const int* list = path_list(*h, subset_num, num_subsets, n, true);
       back_paths(*h, list, n, projdata_dev, projdata_stride, images_dev, image_stride, batch, st, 0);
     } else {
       for (int b = 0; b < batch; ++b)
@@ -224,6 +224,7 @@ int b200rt_log_likelihood_gradient_batch_dev(b200rt_projector* h, const float* i
     ep.small_value = batch_thresholds(*h, y_dev, y_stride, batch, subset_num, num_subsets, zero_seg0_end_planes, st,
                                       ep.sv_stride);
     forward_paths(*h, list, n, images_dev, image_stride, h->ratio_batch.p, pd_size(*h), batch, st, &ep);
+    list = path_list(*h, subset_num, num_subsets, n, true);
     back_paths(*h, list, n, h->ratio_batch.p, pd_size(*h), gradients_dev, gradient_stride, batch, st, 0);
     return B200RT_OK;
   } catch (const std::exception& e) {

@@ -673,12 +673,17 @@ const int* subset_list(b200rt_projector& h, int subset, int nsub, int& count) {
   return p;
 }
 
-// path items (column-staged kernels) of a subset: those whose basic view v has v mod nsub == subset
-const int* path_list(b200rt_projector& h, int subset, int nsub, int& count) {
+// path items of a subset: those whose basic view v has v mod nsub == subset.  Both orders are made at the first call, so that
+// a projection of one direction prepares the other's for a captured stream.
+const int* path_list(b200rt_projector& h, int subset, int nsub, int& count, bool back) {
   const auto key = std::make_pair(subset, nsub);
   auto it = h.path_lists.find(key);
   if (it != h.path_lists.end()) {
     count = h.path_counts[key];
+    if (back) {
+      auto b = h.back_lists.find(key);
+      if (b != h.back_lists.end()) return b->second->p;
+    }
     return it->second->p;
   }
   std::vector<int> list;
@@ -691,11 +696,19 @@ const int* path_list(b200rt_projector& h, int subset, int nsub, int& count) {
   }
   auto buf = std::make_unique<DevBuf<int>>();
   buf->upload(list, h.stream);
+  std::vector<int> mixed = list;
+  back_order(h, mixed);
+  std::unique_ptr<DevBuf<int>> other;
+  if (mixed != list) {
+    other = std::make_unique<DevBuf<int>>();
+    other->upload(mixed, h.stream);
+  }
   ck(cudaStreamSynchronize(h.stream), "path list");
   count = static_cast<int>(list.size());
   h.path_counts[key] = count;
-  const int* p = buf->p;
+  const int* p = back && other ? other->p : buf->p;
   h.path_lists[key] = std::move(buf);
+  if (other) h.back_lists[key] = std::move(other);
   return p;
 }
 
@@ -796,7 +809,7 @@ void ensure_colmax(b200rt_projector& h, float* scratch, cudaStream_t st) {
   const bool grouped = !h.use_paths && h.params.tof_w;
   h.colmax.alloc(1);
   int nall = 0;
-  const int* all = h.use_paths ? path_list(h, 0, 1, nall)
+  const int* all = h.use_paths ? path_list(h, 0, 1, nall, true)
                    : grouped   ? tof_group_list(h, 0, 1, nall)
                                : subset_list(h, 0, 1, nall);
   if (!h.use_paths) ck(cudaMemsetAsync(scratch, 0, sizeof(float) * ni, st), "memset");
@@ -816,7 +829,7 @@ void back_project_into(b200rt_projector& h, const float* pd, float* image, int s
   const int64_t ni = g.image_size();
   int n = 0;
   const bool grouped = !h.use_paths && h.params.tof_w;
-  const int* list = h.use_paths ? path_list(h, subset, nsub, n)
+  const int* list = h.use_paths ? path_list(h, subset, nsub, n, true)
                     : grouped   ? tof_group_list(h, subset, nsub, n)
                                 : subset_list(h, subset, nsub, n);
   if (mode == B200RT_BACKPROJECT_ATOMIC) {
@@ -985,6 +998,7 @@ void b200rt_destroy(b200rt_projector* h) {
     h->subset_lists.clear();
     h->subset_views.clear();
     h->path_lists.clear();
+    h->back_lists.clear();
     h->ossps_g.release();
     h->ossps_pg.release();
     h->ones.release();
@@ -1101,6 +1115,7 @@ int b200rt_set_view_shard(b200rt_projector* h, const int32_t* views, int num_vie
     h->subset_lists.clear();
     h->subset_counts.clear();
     h->path_lists.clear();
+    h->back_lists.clear();
     h->path_counts.clear();
     h->subset_views.clear();
     h->subset_view_counts.clear();

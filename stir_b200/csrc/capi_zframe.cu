@@ -114,6 +114,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   std::vector<ZItemDev> items;
   std::vector<int> item_view, item_out_view;
   std::vector<char> item_lead;  // the first item of a (path, T)
+  std::vector<int> item_block;
   std::vector<PathItemDev> path_items;
   std::vector<char> led(static_cast<size_t>(ntangs));
   std::vector<int> base(ngroups), path0(ngroups);
@@ -222,6 +223,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
               items.push_back(it);
               item_view.push_back(bviews[vi]);
               item_lead.push_back(!led[ti]);
+              item_block.push_back(t0 / kZWarps);
               led[ti] = 1;
               item_out_view.push_back(ov);
               PathItemDev pi{};
@@ -269,6 +271,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
   h.z_work.alloc(items.size());
   h.z_partials.alloc(items.size());
   h.h_item_lead = std::move(item_lead);
+  h.h_item_block = std::move(item_block);
   h.h_item_view = std::move(item_view);
   h.h_item_out_view = std::move(item_out_view);
   h.h_path_items = std::move(path_items);
@@ -429,6 +432,28 @@ void forward_paths(b200rt_projector& h, const int* list, int n, const float* ima
       ck(launch_forward_z(h.params, z, list, n, sp, x, img_stride, 0, o, out_stride, nb, st, &e), "forward projection");
     }
   }
+}
+
+// The order of a back projection's items.  As built, the paths through the middle come first: the longest, and the ones that add
+// most to a voxel, whose float sum is then large, and rounds coarsely, while the many small values of the outer paths come
+// (images of projected phantoms: 7 to 17 % more rounding error than in an order without a preference).  Where the items run in
+// many waves, the blocks of tangential positions take turns (bit-reversed) up to the outer quarter, whose short paths stay last
+// to even out the end (all clinical lines 3.64 ms in either order; 24102 items of 162 records 175 / 188 us).  Error against the
+// fixed-point sums, longest first / in turns, over the column-staged kernels': 1.09 / 1.03 (344 x 344 x 127), 1.10 / 1.02 (171 x 171 x
+// 63), 1.17 / 1.03 (332 x 336 x 11).  Calls of few waves, which have few terms a voxel, keep the longest first (4158 items of 68
+// records: 26 us, in turns 30).
+void back_order(const b200rt_projector& h, std::vector<int>& items) {
+  if (!h.use_z || items.empty() || static_cast<int64_t>(items.size()) < 4 * z_resident_warps(h.zparams, false)) return;
+  const int blocks = *std::max_element(h.h_item_block.begin(), h.h_item_block.end()) + 1, inner = blocks - blocks / 4;
+  int bits = 0;
+  while (1 << bits < inner) ++bits;
+  std::vector<int> turn(blocks);
+  for (int b = 0; b < blocks; ++b) {
+    turn[b] = b < inner ? 0 : (1 << bits) + b;
+    for (int k = 0; b < inner && k < bits; ++k) turn[b] |= (b >> k & 1) << (bits - 1 - k);
+  }
+  std::stable_sort(items.begin(), items.end(),
+                   [&](int a, int b) { return turn[h.h_item_block[a]] < turn[h.h_item_block[b]]; });
 }
 
 // Memory of the call's own where its reductions go to padded columns or to several images, which collect() adds up.
