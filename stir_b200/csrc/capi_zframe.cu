@@ -300,8 +300,9 @@ namespace {
 // records 42 / 22 / 13.5 / 10.4 / 10.3; 438 of 83 30 / 18 / 12.4 / 10.4 / 16.5; 630 of 146 37 / 21 / 13.5 / 16.5 / 23; 1972 of 173
 // 45 / 27 / 27 / 37; 3423 of 391 97 / 72 / 66 / 80; 4158 of 68 27 / 29 / 33; 15892 of 355 282 / 268 / 288; 49350 of 49 196 / 243.
 // Back: 243 of 241 70 / 41 / 27 / 19 / 16.5; 833 of 175 53 / 33 / 24 / 21 / 25; 2618 of 65 28 / 20 / 22 / 28; 4158 of 68 26 / 27 / 30.
-// `far`: also worth it where each warp's own latency is what bounds it (long paths, few registers)
-int sharing_warps(int n, int rec, int resident, bool far) {
+// `far`: also worth it where each warp's own latency is what bounds it (long paths, few registers); `heavy`: not for short parts
+// where a warp's set-up and sums are long (four planes a lane, 1764 items of 39 records: 34 / 41)
+int sharing_warps(int n, int rec, int resident, bool far, bool heavy) {
   int parts = 1;
   while (parts < kZManyWarps) {
     const int next = 2 * parts;
@@ -309,7 +310,7 @@ int sharing_warps(int n, int rec, int resident, bool far) {
     const int r = rec / next;
     const bool ok = m <= 1.0                ? r >= 5
                     : next >= 8             ? false
-                    : m <= 1.5              ? r >= 16
+                    : m <= 1.5              ? r >= (heavy ? 30 : 16)
                     : m <= 2.3              ? r >= 30
                     : far && m <= 4.0       ? r >= 90
                     : far && m <= 12.0      ? next == 2 && r >= 125
@@ -330,20 +331,22 @@ constexpr int kSharedLimit = 200 * 1024;
 // 1.1e-7; 171 x 171 x 63 9.7e-8 / 6.1e-8; 101 x 92 x 23 7.2e-8 / 4.9e-8; short paths (34 x 34 x 41) 7.2e-8 / 4.8e-8 with 8 columns
 // (16: 5.2e-8).  The column-staged kernels, which add the sums of 58 columns by eight warps: 1.0e-7, 2.1e-7, 6.9e-8, 5.7e-8,
 // 5.3e-8.  Steep paths of medium length need four segments (two: 1.2e-7 in the first case).  A segment costs 1 to 2 % of the time
-// (all clinical lines: 4.41 ms with one segment in products of 32, 4.71 with four in products of 16).
+// (all clinical lines: 4.41 ms with one segment in products of 32, 4.53 as here, 4.71 with four segments), 7 % on paths of 123
+// records.
 ZSplit z_split(const b200rt_projector& h, int n) {
   const ZParams& z = h.zparams;
   ZSplit sp;
-  sp.parts = sharing_warps(n, z.mean_rec, z_resident_warps(z, true), z.planes == 1 || (z.planes == 2 && z.nm == 4));
+  sp.parts = sharing_warps(n, z.mean_rec, z_resident_warps(z, true), z.planes == 1 || (z.planes == 2 && z.nm == 4),
+                           z.planes == 4);
   // 16 warps a CTA: two CTAs an SM where the registers allow it, one elsewhere
   if (sp.parts == 16 && n > 148 && (z.nm > 4 || z.planes == 4)) sp.parts = 8;
   while (sp.parts > 1 && std::max(sp.parts, kZWarps) * z_forward_smem(z, 2) > kSharedLimit) sp.parts /= 2;
-  sp.segs = std::max(sp.parts, z.planes == 4 && z.mean_rec >= 64 && z.mean_rec < 256 ? 4 : 2);
+  sp.segs = std::max(sp.parts, z.planes == 4 && z.mean_rec >= 128 && z.mean_rec < 256 ? 4 : 2);
   sp.fold = z.planes > 1 && z.mean_rec < 64 ? 1 : 2;
   return sp;
 }
 int z_back_parts(const b200rt_projector& h, int n) {
-  return sharing_warps(n, h.zparams.mean_rec, z_resident_warps(h.zparams, false), h.zparams.planes == 1);
+  return sharing_warps(n, h.zparams.mean_rec, z_resident_warps(h.zparams, false), h.zparams.planes == 1, false);
 }
 
 // Whether a call is worth padded images, which save instructions and cache lines per column walked and cost a pass over the
