@@ -33,9 +33,9 @@ int lm_check(b200rt_projector* h, const b200rt_lm_event* ev, int64_t n, const fl
 }
 
 // binned (projection kernels over the subset) or per event (one row walk per event): automatically binned once
-// the events number at least 1/16 of the bins, where two whole-subset projections cost less than the events'
-// rows (on the clinical geometry a forward plus a back projection take ~0.4 ns per bin, a row walk ~5 ns per
-// event)
+// the events number at least 1/16 of all bins.  The line is from projections that took ~0.4 ns per bin on the clinical
+// geometry, a row walk ~4-5 ns per event; the present ones take 0.11 ns, so on one subset the methods break even with far
+// fewer events (b200rt_listmode_set_method chooses)
 bool lm_binned(const b200rt_projector& h, int64_t n) {
   if (h.lm_method == B200RT_LISTMODE_PER_EVENT) return false;
   if (h.lm_method == B200RT_LISTMODE_BINNED) return n > 0;

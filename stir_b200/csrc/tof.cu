@@ -17,7 +17,7 @@
 // fixed-point sum, 8e-7 against 1.3e-6; but the result moves by as much as the present error.)
 //
 // 33 timing bins, 8 rings x 288 detectors, all 19.5 M TOF bins: forward 3.59 -> 0.92 ms, back 3.19 -> 1.62 ms.  The weights
-// are read once a projection: 2.9 GB, 0.45 ms at the copy bandwidth.  Both are bound by shared memory (80 and 96 % of the
+// are read once a projection: 2.9 GB, 0.45 ms at the copy bandwidth.  Both are bound by shared memory (77 and 95 % of the
 // l1tex data path): the weights' 16-byte reads, the staged voxels and the groups' sums.
 #include <cstdint>
 

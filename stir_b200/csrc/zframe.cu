@@ -13,10 +13,11 @@
 //            register renaming), and G_m starts again at w2 c;
 //   back:    E_m = the two lines' data of chain m, from shared memory; u = sum_m w E_m is added to the image column.
 //
-// Clinical scanner (72.6 M lines, 344 x 344 x 127 image), all lines: forward 9.20 -> 4.50 ms, back 10.07 -> 3.61
-// ms, deterministic back of one of 7 subsets 1.67 -> 1.02 ms.  Both are bound by latency and issue: 65
-// (forward) and 70 instructions a column against 24 packed multiply-adds a pair of planes cannot do without, 42 - 45 % of
-// the issue slots, 16 and 24 warps per SM (the registers and the data in shared memory).  Tried: two warps per forward item
+// Clinical scanner (72.6 M lines, 344 x 344 x 127 image), all lines: forward 9.20 -> 4.53 ms, back 10.07 -> 3.64
+// ms, deterministic back of one of 7 subsets 1.67 -> 1.02 ms.  Both are bound by latency and issue: 87 (forward) and 90
+// instructions a column, of which the 12 packed multiply-adds (6 chains, 4 planes a lane) cannot be done without; 48 and 53 %
+// of the issue slots, the l1tex data pipe below half and L2 below a fifth of their peaks, 16 and 20 warps per SM (the
+// registers and the data in shared memory).  Tried: two warps per forward item
 // with three chains each (80 registers, 24 warps: 66 % of the slots, but nearly twice the instructions, 6.3 ms); more
 // registers per thread (12 warps: 6.0 ms); data in registers in the back projection too, moved at the events (4.8 ms).
 #include <cstddef>
