@@ -1075,7 +1075,10 @@ cudaError_t launch_back_z_fixed(const ProjParams& p, const ZParams& z, const int
 
 int z_forward_smem(const ZParams& z, int buffers) { return forward_smem(z, buffers); }
 int z_resident_warps(const ZParams& z, bool forward) {
-  return 148 * kZWarps * (forward ? forward_ctas(z.nm, z.planes) : back_ctas(z.planes));
+  // (as compiled, or as many as an SM's 227 KB hold: the clinical back projection's data leave room for 5 CTAs of 6)
+  const int smem = kZWarps * (forward ? forward_smem(z, 1) : back_smem(z)) + 1024;
+  const int fit = 227 * 1024 / smem, compiled = forward ? forward_ctas(z.nm, z.planes) : back_ctas(z.planes);
+  return 148 * kZWarps * (fit < 1 ? 1 : fit < compiled ? fit : compiled);
 }
 
 int z_batch_smem(const ZParams& z, bool forward, int buffers) {
