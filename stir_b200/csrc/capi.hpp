@@ -209,7 +209,7 @@ bool build_zframe(b200rt_projector& h, const std::vector<RowElem>& hr, const std
                   int nsegs, int ntangs, const std::vector<int>& bviews);
 // how a call's n items are walked (zframe.hpp)
 ZSplit z_split(const b200rt_projector& h, int n);
-int z_back_parts(const b200rt_projector& h, int n);
+int z_back_parts(const b200rt_projector& h, int n, int images);
 // path-item projections of a list of items for a batch of images (use_paths).  n_call: the items of the whole call where
 // the list is a part of it (-1: the list is)
 void forward_paths(b200rt_projector& h, const int* list, int n, const float* images, int64_t img_stride, float* out,

@@ -345,8 +345,9 @@ ZSplit z_split(const b200rt_projector& h, int n) {
   sp.fold = z.planes > 1 && z.mean_rec < 64 ? 1 : 2;
   return sp;
 }
-int z_back_parts(const b200rt_projector& h, int n) {
-  return sharing_warps(n, h.zparams.mean_rec, z_resident_warps(h.zparams, false), h.zparams.planes == 1, false);
+int z_back_parts(const b200rt_projector& h, int n, int images) {
+  const int items = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(n) * images, 1 << 30));
+  return sharing_warps(items, h.zparams.mean_rec, z_resident_warps(h.zparams, false), h.zparams.planes == 1, false);
 }
 
 // Whether a call is worth padded images, which save instructions and cache lines per column walked and cost a pass over the
@@ -480,7 +481,7 @@ void BackSums::clear(int images) {
 }
 void BackSums::add(const int* list, int n, const float* pd, int64_t pd_stride, int images, int zero_ends) {
   if (n > 0)
-    ck(launch_back_z(h_.params, h_.zparams, list, n, z_back_parts(h_, n), pd, pd_stride, sums_, per_, h_.zparams.copies,
+    ck(launch_back_z(h_.params, h_.zparams, list, n, z_back_parts(h_, n, images), pd, pd_stride, sums_, per_, h_.zparams.copies,
                      stride_ != h_.params.nz, images, st_, zero_ends),
        "back projection");
 }
@@ -513,7 +514,7 @@ void add_back_paths(b200rt_projector& h, const int* list, int n, const float* pd
                     int64_t img_stride, int batch, cudaStream_t st, int zero_ends) {
   if (n <= 0) return;
   if (h.use_z)
-    ck(launch_back_z(h.params, h.zparams, list, n, z_back_parts(h, n), pd, pd_stride, images, img_stride, 1, 0, batch, st,
+    ck(launch_back_z(h.params, h.zparams, list, n, z_back_parts(h, n, batch), pd, pd_stride, images, img_stride, 1, 0, batch, st,
                      zero_ends),
        "back projection");
   else
@@ -524,7 +525,7 @@ void add_back_paths(b200rt_projector& h, const int* list, int n, const float* pd
 void back_paths_fixed(b200rt_projector& h, const int* list, int n, const float* pd, unsigned long long* acc,
                       const double* scale, cudaStream_t st, int zero_ends) {
   if (h.use_z)
-    ck(launch_back_z_fixed(h.params, h.zparams, list, n, z_back_parts(h, n), pd, acc, scale, st, zero_ends), "back projection");
+    ck(launch_back_z_fixed(h.params, h.zparams, list, n, z_back_parts(h, n, 1), pd, acc, scale, st, zero_ends), "back projection");
   else
     ck(launch_back_paths_fixed(h.params, h.pparams, list, n, pd, acc, scale, st, zero_ends), "back projection");
 }
